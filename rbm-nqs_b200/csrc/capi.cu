@@ -327,6 +327,12 @@ struct rbmnqs_handle {
     DevBuf<double> cgm_t1;
     rbmnqs::CgMultiScratch cgms{};
     int cgm_blocks = 0;
+    // the same for a basic RBM without Pfaffian factor, whose solver works on
+    // the factors of O (cg_factored.cu)
+    bool fact_cg = false;
+    DevBuf<rbmnqs::CgFactProb> cgf;
+    unsigned char* cgf_work = nullptr;  // its partial products, behind the vectors in mfbuf
+    rbmnqs::CgFactScratch cgfs{};
     DevBuf<unsigned char> mfbuf;
     // direct solver above the formed-S sizes: the sample-space (Woodbury) work
     DevBuf<unsigned char> wbbuf;
@@ -679,6 +685,30 @@ struct rbmnqs_handle {
         p.max_it = cg_max_it();
         return p;
     }
+    rbmnqs::CgFactProb cg_fact_prob() const {
+        rbmnqs::CgFactProb p{};
+        p.O = O.p;
+        p.spins = samples.p;
+        p.d = d.p;
+        p.F = F.p;
+        p.x = x.p;
+        p.diag = diag.p;
+        p.max_diag = maxdiag.p;
+        p.sch = sched.p;
+        p.res = cgres.p;
+        p.r = mfw.r;
+        p.p = mfw.p;
+        p.norm = (double)N;
+        p.rtol = cg_rtol();
+        p.N = N;
+        p.P = P;
+        p.n = n;
+        p.nh = nh;
+        p.n_neural = P_neural;
+        p.max_it = cg_max_it();
+        rbmnqs::cg_fact_carve(&p, cgf_work);
+        return p;
+    }
     // a batch solves this session's system in its merged launch: the SR
     // step (not SGD, not the two solves of Heun) by matrix-free CG
     bool batch_cg() const { return multi_cg && cfg.plugin != 3 && cfg.optimizer_type == 0 && !full; }
@@ -731,6 +761,8 @@ struct rbmnqs_handle {
                 ck(rbmnqs::launch_woodbury_solve(O.p, fp64, dS, N, P, P_neural, (double)N, F.p, x.p, maxdiag.p,
                                                  sched.p, 0, 0, 0, wbw, cgres.p, st),
                    "direct solve (sample space)");
+            else if (fact_cg)
+                ck(rbmnqs::launch_cg_fact(cgf.p, 1, fp64, cgfs, cgm_blocks, st), "matrix-free cg");
             else if (multi_cg)
                 ck(rbmnqs::launch_cg_multi(cgm.p, 1, fp64, cgms, cgm_blocks, st), "matrix-free cg");
             else
@@ -1181,11 +1213,17 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
             h->dsync.alloc(1);
             h->dwork.alloc(h->P);
         }
+        h->multi_cg = h->mfree && cfg->solver == 0;
+        // O of a basic RBM has rank-one blocks (spins x activations); the
+        // Pfaffian columns and the centred O of full enumeration do not
+        h->fact_cg = h->multi_cg && cfg->rbm_type == 0 && !h->pf_n && !h->full && h->n <= 128;
         if (h->mfree || h->coop_dense) {
             const int nn = h->mfree ? h->N : 1;
             ck(rbmnqs::mfree_plan(nn, h->P, &h->mfp), "cooperative CG plan");
-            h->mfbuf.alloc(rbmnqs::mfree_work_bytes(nn, h->P, h->mfp));
+            const size_t vec = (rbmnqs::mfree_work_bytes(nn, h->P, h->mfp) + 255) & ~size_t(255);
+            h->mfbuf.alloc(vec + (h->fact_cg ? rbmnqs::cg_fact_work_bytes(nn, n, nh) : 0));
             h->mfw = rbmnqs::mfree_carve(h->mfbuf.p, nn, h->P, h->mfp);
+            h->cgf_work = h->mfbuf.p + vec;
             h->mfw.minres = cfg->solver == 1;
         }
         if (h->mfree) {
@@ -1210,7 +1248,6 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
         h->maxdiag.alloc(1);
         h->sched.alloc(1);
         h->cgres.alloc(1);
-        h->multi_cg = h->mfree && cfg->solver == 0;
         {
             require(cfg->optimizer_type == 0 || cfg->optimizer_type == 1, "optimizer.type must be 0 (SR) or 1 (SGD)");
             require(cfg->plugin >= 0 && cfg->plugin <= 3,
@@ -1340,7 +1377,20 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
             while (h->wpb > 1 && rbmnqs::eval_smem_bytes(h->machine(), h->fp64, h->wpb, pl) > 200 * 1024)
                 h->wpb >>= 1;
         }
-        if (h->multi_cg) {
+        if (h->fact_cg) {
+            rbmnqs::CgFactProb pr = h->cg_fact_prob();
+            const int tiles = rbmnqs::cg_fact_units(&pr, 1, &h->cgfs);
+            h->cgf.alloc(1);
+            h->cgm_t2.alloc(tiles);
+            h->cgm_t1.alloc(2 * (size_t)tiles);
+            ck(cudaMemcpyAsync(h->cgf.p, &pr, sizeof(pr), cudaMemcpyHostToDevice, h->st), "copy");
+            h->cgfs.tdb = h->cgm_t2.p;
+            h->cgfs.tfb = h->cgm_t1.p;
+            h->cgfs.trs = h->cgm_t1.p + tiles;
+            h->cgfs.sync = h->mfw.sync;
+            ck(rbmnqs::cg_fact_blocks(&h->cgm_blocks), "factored CG plan");
+            ck(cudaStreamSynchronize(h->st), "sync");  // pr leaves scope
+        } else if (h->multi_cg) {
             rbmnqs::CgMultiProb pr = h->cg_prob();
             long long rc = 0, tc = 0;
             const int tiles = rbmnqs::cg_multi_units(&pr, 1, &rc, &tc);
@@ -2234,18 +2284,21 @@ struct rbmnqs_batch {
     cudaGraphExec_t graph = nullptr;
     int graph_kernels = 0;
     // sessions whose matrix-free CG runs in the merged multi-system launches
-    // (one launch per precision and per kCgMultiMax systems)
+    // (one launch per precision, per form of the operator and per
+    // kCgMultiMax systems)
     std::vector<char> merged;
     struct Group {
-        int fp64, nprob;
+        int fp64, nprob, fact;
         DevBuf<rbmnqs::CgMultiProb> probs;
+        DevBuf<rbmnqs::CgFactProb> fprobs;
+        rbmnqs::CgFactScratch fsc{};
         DevBuf<double2> t2;
         DevBuf<double> t1;
         DevBuf<rbmnqs::MfreeSync> sync;
         rbmnqs::CgMultiScratch sc{};
     };
     std::vector<std::unique_ptr<Group>> groups;
-    int cg_blocks = 0;
+    int cg_blocks = 0, fact_blocks = 0;
     // sessions whose sweeps run in the batch's sweep launches (one per
     // entries-per-lane class with at least two sessions)
     std::vector<char> swept;
@@ -2292,16 +2345,42 @@ int rbmnqs_batch_create(rbmnqs_handle* const* sessions, int32_t n, rbmnqs_batch*
         for (auto& e : b->joins) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
         for (auto& e : b->cg_done) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
         for (auto& e : b->joins2) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-        // matrix-free CG systems of the same precision share launches when
-        // there are at least two of them
+        // matrix-free CG systems of the same precision and operator form
+        // share launches when there are at least two of them
         b->merged.assign(n, 0);
-        for (int fp = 0; fp < 2; fp++) {
+        for (int kind = 0; kind < 4; kind++) {
+            const int fp = kind & 1, fact = kind >> 1;
             std::vector<int> idx;
             for (int i = 0; i < n; i++)
-                if (b->hs[i]->batch_cg() && b->hs[i]->fp64 == fp) idx.push_back(i);
+                if (b->hs[i]->batch_cg() && b->hs[i]->fp64 == fp && b->hs[i]->fact_cg == (fact != 0)) idx.push_back(i);
             if (idx.size() < 2) continue;
             for (size_t g0 = 0; g0 < idx.size(); g0 += rbmnqs::kCgMultiMax) {
                 auto g = std::make_unique<rbmnqs_batch::Group>();
+                g->fact = fact;
+                g->sync.alloc(1);
+                if (fact) {
+                    std::vector<rbmnqs::CgFactProb> pr;
+                    for (size_t k = g0; k < std::min(idx.size(), g0 + rbmnqs::kCgMultiMax); k++) {
+                        pr.push_back(b->hs[idx[k]]->cg_fact_prob());
+                        b->merged[idx[k]] = 1;
+                    }
+                    g->fp64 = fp;
+                    g->nprob = (int)pr.size();
+                    const int tiles = rbmnqs::cg_fact_units(pr.data(), g->nprob, &g->fsc);
+                    g->fprobs.alloc(pr.size());
+                    g->t2.alloc(tiles);
+                    g->t1.alloc(2 * (size_t)tiles);
+                    ck(cudaMemcpyAsync(g->fprobs.p, pr.data(), pr.size() * sizeof(rbmnqs::CgFactProb),
+                                       cudaMemcpyHostToDevice, b->st),
+                       "copy");
+                    ck(cudaStreamSynchronize(b->st), "sync");  // pr leaves scope
+                    g->fsc.tdb = g->t2.p;
+                    g->fsc.tfb = g->t1.p;
+                    g->fsc.trs = g->t1.p + tiles;
+                    g->fsc.sync = g->sync.p;
+                    b->groups.push_back(std::move(g));
+                    continue;
+                }
                 std::vector<rbmnqs::CgMultiProb> pr;
                 for (size_t k = g0; k < std::min(idx.size(), g0 + rbmnqs::kCgMultiMax); k++) {
                     pr.push_back(b->hs[idx[k]]->cg_prob());
@@ -2314,7 +2393,6 @@ int rbmnqs_batch_create(rbmnqs_handle* const* sessions, int32_t n, rbmnqs_batch*
                 g->probs.alloc(pr.size());
                 g->t2.alloc(2 * (size_t)tiles);
                 g->t1.alloc(tiles);
-                g->sync.alloc(1);
                 ck(cudaMemcpyAsync(g->probs.p, pr.data(), pr.size() * sizeof(rbmnqs::CgMultiProb),
                                    cudaMemcpyHostToDevice, b->st),
                    "copy");
@@ -2327,7 +2405,10 @@ int rbmnqs_batch_create(rbmnqs_handle* const* sessions, int32_t n, rbmnqs_batch*
                 b->groups.push_back(std::move(g));
             }
         }
-        if (!b->groups.empty()) ck(rbmnqs::cg_multi_blocks(&b->cg_blocks), "multi-system CG plan");
+        for (const auto& g : b->groups) {
+            if (g->fact && !b->fact_blocks) ck(rbmnqs::cg_fact_blocks(&b->fact_blocks), "factored CG plan");
+            if (!g->fact && !b->cg_blocks) ck(rbmnqs::cg_multi_blocks(&b->cg_blocks), "multi-system CG plan");
+        }
         // sweeps: the plain FP32 Metropolis sessions grouped by entries per lane
         b->swept.assign(n, 0);
         b->sweep_group.assign(n, -1);
@@ -2413,7 +2494,8 @@ int rbmnqs_batch_epoch(rbmnqs_batch* b, rbmnqs_sample_stats* s, rbmnqs_sr_stats*
                     // sample and var(O) (and after the other cooperative
                     // solves), then each merged session's update
                     for (auto& g : b->groups)
-                        ck(rbmnqs::launch_cg_multi(g->probs.p, g->nprob, g->fp64, g->sc, b->cg_blocks, b->st),
+                        ck(g->fact ? rbmnqs::launch_cg_fact(g->fprobs.p, g->nprob, g->fp64, g->fsc, b->fact_blocks, b->st)
+                                   : rbmnqs::launch_cg_multi(g->probs.p, g->nprob, g->fp64, g->sc, b->cg_blocks, b->st),
                            "matrix-free cg");
                     ck(cudaEventRecord(b->solved, b->st), "solved");
                     for (size_t i = 0; i < b->hs.size(); i++) {

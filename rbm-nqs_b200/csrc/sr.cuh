@@ -198,6 +198,44 @@ int cg_multi_units(CgMultiProb* probs, int nprob, long long* row_cost, long long
 cudaError_t cg_multi_blocks(int* blocks);
 cudaError_t launch_cg_multi(const CgMultiProb* probs_dev, int nprob, int fp64, const CgMultiScratch& s, int blocks,
                             cudaStream_t st);
+// Matrix-free CG systems of basic RBMs (cg1 semantics) on the factors of O
+// (cg_factored.cu): the samples' spins and the hidden activations in the
+// first n + nh entries of the O rows.  n <= 128 sites, P = n + nh + n nh.
+struct CgFactProb {
+    const void* O;          // [N][P] float2 or double2 (one precision per launch)
+    const uint32_t* spins;  // [N][4] the samples' configurations
+    const double2* d;
+    const double2* F;
+    double2* x;
+    const double* diag;
+    const double* max_diag;
+    const ScheduleDev* sch;
+    CgResultDev* res;
+    double2 *r, *p;  // P entries
+    // partial products (cg_fact_carve): u per hidden tile, Y and |u|^2 per sample chunk
+    double2 *upart, *ypart;
+    double* vv;
+    double norm, rtol;
+    int N, P, n, nh, n_neural, max_it;
+    // filled by cg_fact_units: first unit costs per phase and first tile
+    long long a_cost0, b_cost0, t_cost0;
+    int tile0, pad;
+};
+struct CgFactScratch {
+    double2* tdb;  // per tile: d . b
+    double *tfb, *trs;  // per tile: sum f |b|^2, ||r||^2
+    MfreeSync* sync;
+    long long a_cost, b_cost, t_cost;
+};
+// Work bytes of one system, and their layout into the descriptor.
+size_t cg_fact_work_bytes(int N, int n, int nh);
+void cg_fact_carve(CgFactProb* p, void* base);
+// Fills the unit offsets of the descriptors and the costs of the scratch;
+// returns the total tile count (the length of each partial-sum array).
+int cg_fact_units(CgFactProb* probs, int nprob, CgFactScratch* sc);
+cudaError_t cg_fact_blocks(int* blocks);
+cudaError_t launch_cg_fact(const CgFactProb* probs_dev, int nprob, int fp64, const CgFactScratch& s, int blocks,
+                           cudaStream_t st);
 // The direct solver above the formed-S sizes (woodbury.cu): S_reg x = F
 // through the N x N system K = N I + Abar Lambda^-1 Abar^H of the Woodbury
 // identity, K factored by launch_direct_solve.

@@ -9,9 +9,11 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../host/model.hpp"
@@ -117,6 +119,9 @@ struct TermHost {
     std::vector<rbmnqs::TermDev> terms, diag;
     std::vector<double2> vals;
     int nf_max = 0;
+    // symmetric machines: row tuples (TermTable)
+    std::vector<uint16_t> cls;
+    std::vector<uint8_t> tup;
 };
 
 TermHost build_terms(const std::vector<rbmnqs::local_op>& ops) {
@@ -160,6 +165,38 @@ TermHost build_terms(const std::vector<rbmnqs::local_op>& ops) {
         }
     }
     return t;
+}
+
+// The distinct row tuples of the terms under the symmetries (TermTable),
+// numbered in the order in which the terms' orbits enumerate them, so that
+// consecutive symmetries of a term mostly have consecutive tuples.
+void build_tuples(TermHost* t, const std::vector<std::vector<int>>& perm, int n) {
+    std::vector<int> pairs((size_t)(n + 1) * (n + 1), -1);  // ids of one and two rows
+    std::unordered_map<uint64_t, int> more;                 // of up to six, by the tuple's eight bytes
+    int count = 0;
+    t->cls.reserve(t->terms.size() * perm.size());
+    for (const auto& d : t->terms) {
+        const int nf = (d.flip1 >> 16) & 0xff;
+        for (const auto& p : perm) {
+            uint8_t r[8] = {};
+            for (int q = 0; q < nf; q++)
+                r[q] = (uint8_t)p[q < 4 ? (d.flip0 >> (8 * q)) & 0xff : (d.flip1 >> (8 * (q - 4))) & 0xff];
+            r[6] = (uint8_t)nf;
+            uint64_t key;
+            std::memcpy(&key, r, sizeof(key));
+            int& id = nf <= 2 ? pairs[(size_t)r[0] * (n + 1) + (nf == 2 ? r[1] : n)]
+                              : more.emplace(key, -1).first->second;
+            if (id < 0) {
+                id = count++;
+                t->tup.insert(t->tup.end(), r, r + 8);
+            }
+            t->cls.push_back((uint16_t)std::min(id, 0xffff));
+        }
+    }
+    if (count >= 0xffff) {  // not indexable in 16 bits
+        t->cls.clear();
+        t->tup.clear();
+    }
 }
 
 // Row order of W in the shared memory of the FP32 evaluation kernel
@@ -224,6 +261,8 @@ int rbmnqs::test_fault() { return g_test_fault.load(std::memory_order_relaxed); 
 struct TermBufs {
     DevBuf<rbmnqs::TermDev> terms, diag;
     DevBuf<double2> vals;
+    DevBuf<uint16_t> cls;
+    DevBuf<uint8_t> tup;
     rbmnqs::TermTable tt{};
     void upload(const TermHost& t) {
         terms.alloc(std::max<size_t>(1, t.terms.size()));
@@ -244,6 +283,15 @@ struct TermBufs {
         tt.terms = terms.p;
         tt.diag = diag.p;
         tt.vals = vals.p;
+        if (!t.cls.empty()) {
+            cls.alloc(t.cls.size());
+            tup.alloc(t.tup.size());
+            ck(cudaMemcpy(cls.p, t.cls.data(), t.cls.size() * sizeof(uint16_t), cudaMemcpyHostToDevice), "c");
+            ck(cudaMemcpy(tup.p, t.tup.data(), t.tup.size(), cudaMemcpyHostToDevice), "c");
+            tt.n_cls = (int)t.tup.size() / 8;
+            tt.cls = cls.p;
+            tt.tup = tup.p;
+        }
     }
 };
 
@@ -1136,7 +1184,11 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
         ck(cudaMemcpy(h->rowptr.p, hh.rowptr.data(), hh.rowptr.size() * sizeof(int), cudaMemcpyHostToDevice), "c");
         ck(cudaMemcpy(h->emask.p, hh.mask.data(), hh.mask.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "c");
         ck(cudaMemcpy(h->eval.p, hh.val.data(), hh.val.size() * sizeof(double2), cudaMemcpyHostToDevice), "c");
-        h->terms.upload(build_terms(m.hamiltonian));
+        {
+            TermHost th = build_terms(m.hamiltonian);
+            if (cfg->rbm_type == 1 && n <= 255) build_tuples(&th, m.perm, n);
+            h->terms.upload(th);
+        }
         // observables (evaluation mode), one table each
         for (const auto& op : m.observables) {
             auto od = std::make_unique<ObsDev>();

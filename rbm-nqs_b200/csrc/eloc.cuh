@@ -294,6 +294,77 @@ __device__ __forceinline__ void seg_global(const float2* p, float2 (&r)[KB / 2 >
     }
 }
 
+// The O_k row of a symmetric machine from the warp's scratch: tn = tanh theta
+// [T], sgn = the spins as +-1 [n].
+__device__ __forceinline__ void write_O_sym(const MachineDev& m, const uint32_t (&sp)[4], const float2* tn,
+                                            const float* sgn, const uint8_t* sInv, float2* Orow, int lane) {
+    const int n = m.n, nh = m.nh, S = m.S, n_vb = m.n_vb;
+    // v: sum_s sigma_{P_s(basis_q)}; h: sum_s tanh theta[k, s]
+    for (int q = 0; q < n_vb; q++) {
+        float acc = 0.f;
+        for (int s = lane; s < S; s += 32) acc += sbit(sp, m.orbit[q * S + s]) ? -1.f : 1.f;
+        acc = warp_sum(acc);
+        if (lane == 0) Orow[q] = make_float2(acc, 0.f);
+    }
+    for (int k = 0; k < nh; k++) {
+        float2 acc = make_float2(0.f, 0.f);
+        for (int s = lane; s < S; s += 32) {
+            const float2 v = tn[k + nh * s];
+            acc.x += v.x;
+            acc.y += v.y;
+        }
+        acc.x = warp_sum(acc.x);
+        acc.y = warp_sum(acc.y);
+        if (lane == 0) Orow[n_vb + k] = acc;
+    }
+    // W[j, k]: sum_s sigma_{P_s^{-1}(j)} tanh theta[k, s].  With
+    // n a multiple of 128 and nh of 4, each lane takes four
+    // consecutive sites: one 32-bit load gives their four
+    // inverse-symmetry bytes, two 16-byte loads the four tanh
+    // values they share (same sums, same order per output)
+    if (n % 128 == 0 && nh % 4 == 0) {
+        for (int jb = 4 * lane; jb < n; jb += 128) {
+            for (int k0 = 0; k0 < nh; k0 += 4) {
+                float2 acc[4][4] = {};
+                for (int s = 0; s < S; s++) {
+                    const uint32_t iv = *reinterpret_cast<const uint32_t*>(sInv + s * n + jb);
+                    const float4 t01 = *reinterpret_cast<const float4*>(tn + k0 + nh * s);
+                    const float4 t23 = *reinterpret_cast<const float4*>(tn + k0 + 2 + nh * s);
+                    const float2 t[4] = {make_float2(t01.x, t01.y), make_float2(t01.z, t01.w),
+                                         make_float2(t23.x, t23.y), make_float2(t23.z, t23.w)};
+#pragma unroll
+                    for (int jj = 0; jj < 4; jj++) {
+                        const float sg = sgn[(iv >> (8 * jj)) & 0xffu];
+                        const float2 G2 = make_float2(sg, sg);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) acc[jj][i] = __ffma2_rn(G2, t[i], acc[jj][i]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int jj = 0; jj < 4; jj++)
+                        Orow[n_vb + nh + jb + jj + n * (k0 + i)] = acc[jj][i];
+            }
+        }
+    } else
+    for (int j = lane; j < n; j += 32) {
+        for (int k0 = 0; k0 < nh; k0 += 4) {
+            float2 acc[4] = {};
+            for (int s = 0; s < S; s++) {
+                const float sg = sgn[sInv[s * n + j]];
+                const float2 G2 = make_float2(sg, sg);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (k0 + i < nh) acc[i] = __ffma2_rn(G2, tn[k0 + i + nh * s], acc[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (k0 + i < nh) Orow[n_vb + nh + j + n * (k0 + i)] = acc[i];
+        }
+    }
+}
+
 template <int KB, int NG, bool SYM, int NFM>
 __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* NG))
     eloc_kernel(const EvalArgs a, const ElocLayout L) {
@@ -584,70 +655,7 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
             __syncwarp();
             float2* Orow = reinterpret_cast<float2*>(a.O) + (size_t)b * m.P;
             if (SYM) {
-                // v: sum_s sigma_{P_s(basis_q)}; h: sum_s tanh theta[k, s]
-                for (int q = 0; q < n_vb; q++) {
-                    float acc = 0.f;
-                    for (int s = lane; s < S; s += 32) acc += sbit(sp, m.orbit[q * S + s]) ? -1.f : 1.f;
-                    acc = warp_sum(acc);
-                    if (lane == 0) Orow[q] = make_float2(acc, 0.f);
-                }
-                for (int k = 0; k < nh; k++) {
-                    float2 acc = make_float2(0.f, 0.f);
-                    for (int s = lane; s < S; s += 32) {
-                        const float2 v = tn[k + nh * s];
-                        acc.x += v.x;
-                        acc.y += v.y;
-                    }
-                    acc.x = warp_sum(acc.x);
-                    acc.y = warp_sum(acc.y);
-                    if (lane == 0) Orow[n_vb + k] = acc;
-                }
-                // W[j, k]: sum_s sigma_{P_s^{-1}(j)} tanh theta[k, s].  With
-                // n a multiple of 128 and nh of 4, each lane takes four
-                // consecutive sites: one 32-bit load gives their four
-                // inverse-symmetry bytes, two 16-byte loads the four tanh
-                // values they share (same sums, same order per output)
-                if (n % 128 == 0 && nh % 4 == 0) {
-                    for (int jb = 4 * lane; jb < n; jb += 128) {
-                        for (int k0 = 0; k0 < nh; k0 += 4) {
-                            float2 acc[4][4] = {};
-                            for (int s = 0; s < S; s++) {
-                                const uint32_t iv = *reinterpret_cast<const uint32_t*>(sInv + s * n + jb);
-                                const float4 t01 = *reinterpret_cast<const float4*>(tn + k0 + nh * s);
-                                const float4 t23 = *reinterpret_cast<const float4*>(tn + k0 + 2 + nh * s);
-                                const float2 t[4] = {make_float2(t01.x, t01.y), make_float2(t01.z, t01.w),
-                                                     make_float2(t23.x, t23.y), make_float2(t23.z, t23.w)};
-#pragma unroll
-                                for (int jj = 0; jj < 4; jj++) {
-                                    const float sg = sgn[(iv >> (8 * jj)) & 0xffu];
-                                    const float2 G2 = make_float2(sg, sg);
-#pragma unroll
-                                    for (int i = 0; i < 4; i++) acc[jj][i] = __ffma2_rn(G2, t[i], acc[jj][i]);
-                                }
-                            }
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-#pragma unroll
-                                for (int jj = 0; jj < 4; jj++)
-                                    Orow[n_vb + nh + jb + jj + n * (k0 + i)] = acc[jj][i];
-                        }
-                    }
-                } else
-                for (int j = lane; j < n; j += 32) {
-                    for (int k0 = 0; k0 < nh; k0 += 4) {
-                        float2 acc[4] = {};
-                        for (int s = 0; s < S; s++) {
-                            const float sg = sgn[sInv[s * n + j]];
-                            const float2 G2 = make_float2(sg, sg);
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-                                if (k0 + i < nh) acc[i] = __ffma2_rn(G2, tn[k0 + i + nh * s], acc[i]);
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            if (k0 + i < nh) Orow[n_vb + nh + j + n * (k0 + i)] = acc[i];
-                    }
-                }
+                write_O_sym(m, sp, tn, sgn, sInv, Orow, lane);
             } else {
                 for (int q = lane; q < n_vb; q += 32) Orow[q] = make_float2(sbit(sp, q) ? -1.f : 1.f, 0.f);
                 for (int k = lane; k < nh; k += 32) Orow[n_vb + k] = tn[k];

@@ -117,6 +117,13 @@ struct TermTable {
     const TermDev* terms = nullptr;
     const TermDev* diag = nullptr;
     const double2* vals = nullptr;
+    // symmetric machines: the distinct tuples of W rows (P_s(f_0), P_s(f_1),
+    // ...) that the terms flip under the symmetries s.  cls[t * S + s] is the
+    // tuple of term t and symmetry s, tup[8 c ..] the rows of tuple c and, in
+    // byte 6, their number (null: not built)
+    int n_cls = 0;
+    const uint16_t* cls = nullptr;
+    const uint8_t* tup = nullptr;
 };
 
 struct EvalArgs {
@@ -224,6 +231,11 @@ cudaError_t launch_eval(const EvalArgs& a, int fp64, int warps_per_block, cudaSt
 // factor).  cudaErrorNotSupported when the machine or the table does not fit
 // it; launch_eval then runs eval_kernel.
 cudaError_t launch_eloc_fast(const EvalArgs& a, cudaStream_t st);
+// The same for symmetric machines, psi ratios as products over tables of the
+// distinct flipped row tuples (eloc_sym.cu); cudaErrorNotSupported when the
+// machine is not symmetric or its tables do not fit, launch_eloc_fast then
+// runs its general kernel.
+cudaError_t launch_eloc_sym(const EvalArgs& a, cudaStream_t st);
 int elements_per_lane(int T);
 cudaError_t launch_advance(uint32_t* ctl, int reinit, cudaStream_t st);
 cudaError_t launch_mufu_probe(float* out, int iters, int blocks, cudaStream_t st);

@@ -318,6 +318,7 @@ struct rbmnqs_handle {
 
     DevBuf<double2> params, vb, hb, W64, x;
     DevBuf<float2> W32;
+    DevBuf<float> P32;  // exp(+-4 W) for the screened FP32 sweep
     DevBuf<uint8_t> perm, inv, orbit;
     DevBuf<uint8_t> wrank;  // row order of W in the FP32 evaluation kernel (symmetric machines)
     DevBuf<rbmnqs::OpDev> ops;
@@ -467,6 +468,7 @@ struct rbmnqs_handle {
         m.symmetric = cfg.rbm_type == 1;
         m.W64 = W64.p;
         m.W32 = W32.p;
+        m.P32 = P32.p;
         m.hb = hb.p;
         m.vb = vb.p;
         m.perm = perm.p;
@@ -688,7 +690,7 @@ struct rbmnqs_handle {
             // The sample statistics reported are the first sample's.
             enqueue_solve(cg_after, nullptr, true);
             ck(rbmnqs::launch_heun_begin(params.p, x.p, P, sched.p, cgres.p, plug.p, st), "heun");
-            ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, st), "unpack");
+            ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, P32.p, st), "unpack");
             ck(cudaMemcpyAsync(stats_first.p, stats.p, sizeof(rbmnqs::EpochStatsDev), cudaMemcpyDeviceToDevice, st),
                "copy");
             enqueue_sample(false);
@@ -700,7 +702,7 @@ struct rbmnqs_handle {
                                           cfg.optimizer_type == 0, st),
                "heun");
         }
-        ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, st), "unpack");
+        ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, P32.p, st), "unpack");
         mark(6);
     }
     // the CG limits of cg_solver.cpp:260-334 (cg1)
@@ -770,7 +772,7 @@ struct rbmnqs_handle {
     void enqueue_optimize_post() {
         mark(5);
         ck(rbmnqs::launch_update(params.p, x.p, P, sched.p, cgres.p, plug.p, st), "update");
-        ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, st), "unpack");
+        ck(rbmnqs::launch_unpack(params.p, n, n_vb, nh, vb.p, hb.p, W64.p, W32.p, P32.p, st), "unpack");
         mark(6);
     }
     // solves that are cooperative launches (ordered one after another in a batch graph)
@@ -1352,7 +1354,15 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
         }
         // launch shapes: persistent sampler blocks; evaluation kernels with
         // FP32 W in shared memory when it fits
-        ck(rbmnqs::plan_sampler(h->machine(), h->fp64, cfg->n_chains, h->n_prop_bonds, &h->shape), "sampler plan");
+        ck(rbmnqs::plan_sampler(h->machine(), h->fp64, cfg->n_chains, h->n_prop_bonds, &h->shape, 0, -1,
+                                cfg->proposal == 0),
+           "sampler plan");
+        if (h->shape.plan.screen && !h->full) {
+            h->P32.alloc((size_t)4 * n * nh);
+            // the factors of the zero weights
+            ck(rbmnqs::launch_unpack(h->params.p, n, h->n_vb, nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->P32.p, h->st),
+               "unpack");
+        }
         if (cfg->proposal == 1) {
             // move dictionary: every site, then the Hamiltonian's distinct
             // off-diagonal flip sets of two or more sites
@@ -1481,7 +1491,7 @@ int rbmnqs_set_weights(rbmnqs_handle* h, const double* w) {
     return guard([&] {
         require(h && w, "null argument");
         ck(cudaMemcpyAsync(h->params.p, w, h->P * sizeof(double2), cudaMemcpyHostToDevice, h->st), "copy");
-        ck(rbmnqs::launch_unpack(h->params.p, h->n, h->n_vb, h->nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->st),
+        ck(rbmnqs::launch_unpack(h->params.p, h->n, h->n_vb, h->nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->P32.p, h->st),
            "unpack");
         // a pageable host buffer is free once the copy call returns (the unpack
         // is ordered before any later work on the stream); a pinned or
@@ -2155,7 +2165,8 @@ int rbmnqs_autotune(rbmnqs_handle* h, int32_t sweeps, int32_t* sampler_wpb, int3
                 const int top = std::max(h->shape.warps_per_block, 32);
                 for (int cap = top; cap >= 1; cap /= 2) {
                     rbmnqs::SamplerShape sh{};
-                    ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &sh, cap, pm),
+                    ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &sh, cap, pm,
+                                            !h->net),
                        "sampler plan");
                     if (sh.plan.pair != pm) break;  // two chains per warp not possible here
                     if (std::find(tried.begin(), tried.end(), sh.warps_per_block) != tried.end()) continue;
@@ -2173,7 +2184,7 @@ int rbmnqs_autotune(rbmnqs_handle* h, int32_t sweeps, int32_t* sampler_wpb, int3
             }
             rbmnqs::SamplerShape chk{};
             ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &chk,
-                                    best.warps_per_block, best.plan.pair),
+                                    best.warps_per_block, best.plan.pair, !h->net),
                "sampler plan");
             h->shape = chk;
         }
@@ -2306,7 +2317,7 @@ int rbmnqs_set_sweep_shape(rbmnqs_handle* h, int32_t warps_per_block, int32_t ch
         require(!h->pf_n, "the Pfaffian buffers are sized for the planned shape", RBMNQS_ERR_UNSUPPORTED);
         rbmnqs::SamplerShape sh{};
         ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &sh, warps_per_block,
-                                chains_per_warp == 2 ? 1 : 0),
+                                chains_per_warp == 2 ? 1 : 0, !h->net),
            "sampler plan");
         require(sh.plan.pair == (chains_per_warp == 2),
                 "two chains per warp needs the FP32 expanded-table sweep with n <= 32", RBMNQS_ERR_UNSUPPORTED);
@@ -2839,7 +2850,7 @@ int rbmnqs_load(rbmnqs_handle* h, const char* path) {
         }
         std::fclose(f);
         ck(cudaMemcpyAsync(h->params.p, w.data(), h->P * sizeof(double2), cudaMemcpyHostToDevice, h->st), "copy");
-        ck(rbmnqs::launch_unpack(h->params.p, h->n, h->n_vb, h->nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->st),
+        ck(rbmnqs::launch_unpack(h->params.p, h->n, h->n_vb, h->nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->P32.p, h->st),
            "unpack");
         h->n_updates = (int64_t)nu;
         set_schedules(h, h->n_updates);

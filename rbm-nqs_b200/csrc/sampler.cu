@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "sampler.cuh"
+#include "sweep_common.cuh"
 
 namespace rbmnqs {
 
@@ -29,48 +30,6 @@ template <> struct Wsel<float> {
 template <> struct Wsel<double> {
     static __device__ __forceinline__ const double2* get(const MachineDev& m, const float2*) { return m.W64; }
 };
-
-// Shared-memory loads by 32-bit shared address: the gather tables may also
-// live in global memory, so their generic pointers would otherwise compile
-// to generic loads.
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ float2 lds_f2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds_u8(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-// N / 4 words from a 4 N-byte aligned shared address (N = 4, 8, 16)
-template <int N> __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[N / 4]) {
-    if constexpr (N == 16) {
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
-    } else if constexpr (N == 8) {
-        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(addr));
-    } else {
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[0]) : "r"(addr));
-    }
-}
-
-// word i of the configuration with constant indices only (a runtime index
-// would place the array in local memory)
-__device__ __forceinline__ uint32_t spin_word(const uint32_t sp[4], int i) {
-    return i == 0 ? sp[0] : (i == 1 ? sp[1] : (i == 2 ? sp[2] : sp[3]));
-}
-__device__ __forceinline__ int spin_bit(const uint32_t sp[4], int i) {
-    const uint32_t w = i < 32 ? sp[0] : (i < 64 ? sp[1] : (i < 96 ? sp[2] : sp[3]));
-    return (w >> (i & 31)) & 1;
-}
-__device__ __forceinline__ void flip_bit(uint32_t sp[4], int i) {
-    const uint32_t b = 1u << (i & 31);
-    if (i < 32) sp[0] ^= b;
-    else if (i < 64) sp[1] ^= b;
-    else if (i < 96) sp[2] ^= b;
-    else sp[3] ^= b;
-}
 
 // Lane `lane` owns theta entries t = lane + 32 e (e < E), t = k + nh*s.
 __device__ __forceinline__ bool slot_valid(int lane, int e, int T) { return lane + 32 * e < T; }
@@ -620,57 +579,12 @@ __device__ inline void load_tables(const MachineDev& m, const Smem& s, int fp64,
     __syncthreads();
 }
 
-// Initial configuration of a chain: Philox stream 1 bits for a fresh chain,
-// else the persisted configuration.
-__device__ __forceinline__ void chain_start(const SamplerArgs& a, int chain, uint2 key, uint32_t epoch, uint32_t sp[4]) {
-    const int n = a.m.n;
-    if (a.ctl[1] && a.sweep0 == 0) {
-        const uint4 r = philox4x32(make_uint4(0, epoch, (uint32_t)chain, 1), key);
-        const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            const int lo = 32 * w;
-            const uint32_t mask = n >= lo + 32 ? 0xffffffffu : (n > lo ? ((1u << (n - lo)) - 1) : 0u);
-            sp[w] = rw[w] & mask;
-        }
-    } else {
-#pragma unroll
-        for (int w = 0; w < 4; w++) sp[w] = a.spins[4 * chain + w];
-    }
-}
-
-// Proposal counter at the start of a segment: 32-aligned (proposals are
-// drawn 32 at a time) and past every proposal of earlier segments (a sweep
-// makes at most n proposals).
-__device__ __forceinline__ uint32_t prop_base(const SamplerArgs& a) {
-    return (uint32_t)a.sweep0 * (uint32_t)(32 * ((a.m.n + 31) / 32));
-}
-__device__ __forceinline__ int segment_sweeps(const SamplerArgs& a) {
-    return a.nsweeps ? a.nsweeps : a.spc * a.step + a.warmup;
-}
-// sample slot of global sweep sg, or -1
-__device__ __forceinline__ int sample_slot(const SamplerArgs& a, int st) {
-    const int sg = a.sweep0 + st;
-    if (!a.record || sg < a.warmup || (sg - a.warmup) % a.step) return -1;
-    return (sg - a.warmup) / a.step;
-}
-
 // theta_out[chain][lane + 32 e] = th[e] (coalesced per e)
 template <int E>
 __device__ __forceinline__ void store_theta(float2* out, int chain, int lane, const float2 (&th)[E]) {
     float2* dst = out + (size_t)chain * (32 * E) + lane;
 #pragma unroll
     for (int e = 0; e < E; e++) dst[32 * e] = th[e];
-}
-
-__device__ __forceinline__ void chain_finish(const SamplerArgs& a, int chain, int lane, const uint32_t sp[4],
-                                             uint32_t nacc, uint32_t prop) {
-    if (lane < 4) a.spins[4 * chain + lane] = spin_word(sp, lane);
-    if (lane == 0) {
-        const uint32_t made = prop - prop_base(a);
-        a.n_acc[chain] = (a.sweep0 ? a.n_acc[chain] : 0u) + nacc;
-        a.n_prop[chain] = (a.sweep0 ? a.n_prop[chain] : 0u) + made;
-    }
 }
 
 // One chain: metropolis_sampler::sample_chain (metropolis_sampler.cpp:118-273)
@@ -855,22 +769,6 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Smem& sm, 
 // flushed z (|a| > 43) leaves m2 = 1, the exact limit; a flushed m2 (a zero
 // of cosh to FP32 precision) gives ln|cosh| = -inf, i.e. a proposal of
 // vanishing amplitude that is rejected either way.
-__device__ __forceinline__ float ex2_ftz(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2_ftz(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float cos_ftz(float x) {
-    float y;
-    asm("cos.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Sum of ln|cosh| (the form above) over a lane's E entries: the |a| terms
 // add up and the factors 1 + z^2 + 2 z cos 2b (each in [0, 4]) multiply in
 // groups of four, one lg2 per group instead of one per entry.  A group's
@@ -895,21 +793,6 @@ template <int E> __device__ __forceinline__ float lnc_sweep_sum(const float2 (&t
         lg += lg2_ftz(pm);
     }
     return fmaf(0.346573590279972655f, lg, sa);
-}
-
-// Sum over the warp of the lanes' ln|cosh| differences for the acceptance
-// test.  The partials are summed as fixed-point integers (2^-22 steps, one
-// redux.sync instead of a five-level shuffle butterfly) when every lane's
-// partial is below 16 in magnitude, which keeps the 32-lane total inside
-// int32; otherwise the FP32 butterfly.  The quantisation (2.4e-7) is that of
-// an FP32 sum of this size, so decisions differ from the FP64 chains only at
-// ties, as with any FP32 sum.
-constexpr float kFixScale = 4194304.f;  // 2^22
-__device__ __forceinline__ int fix22(float v) { return __float2int_rn(v * kFixScale); }
-__device__ __forceinline__ float sweep_sum(float v) {
-    const int isum = __reduce_add_sync(kFull, fix22(v));
-    if (__any_sync(kFull, !(fabsf(v) < 16.f))) return warp_sum(v);
-    return (float)isum * (1.f / kFixScale);
 }
 
 // FP32 sweep path with the expanded flip table in shared memory.  Proposals
@@ -2290,6 +2173,7 @@ static cudaError_t plan_sampler_impl(const MachineDev& m, int fp64, int n_chains
     const int budget = smem_max - 8 * 1024;
     const int TP = 32 * E;
     SmemPlan pl{};
+    pl.lane_entries = E;
     // FP32 expanded-table path when the table fits; its theta recompute uses
     // the FP64 expanded table when that fits too, else FP64 W
     const int pf = m.pf.n > 0;
@@ -2364,8 +2248,16 @@ static cudaError_t plan_sampler_impl(const MachineDev& m, int fp64, int n_chains
     return cudaSuccess;
 }
 
+// screen false: not the screened sweep for FP32 sessions, whose start (z of every
+// entry) a launch of few sweeps does not earn back (learned moves between
+// sweeps, 8192 chains of 128 spins: 6.8 ms of sweep stage by the exact sums, 8.0
+// screened).
 cudaError_t plan_sampler(const MachineDev& m, int fp64, int n_chains, int n_bonds, SamplerShape* out, int max_wpb,
-                         int pair_mode) {
+                         int pair_mode, bool screen) {
+    cudaError_t err = cudaSuccess;
+    if (m.pf.n == 0 && (fp64 || (screen && pair_mode != 1)) &&
+        plan_screen(m, fp64, n_chains, n_bonds, max_wpb, out, &err))
+        return err;
     return plan_sampler_impl(m, fp64, n_chains, n_bonds, out, max_wpb, pair_mode);
 }
 
@@ -2388,12 +2280,13 @@ cudaError_t ensure_dynamic_smem(const void* fn, int bytes) {
 // The FP32 expanded-table (one chain per warp) and gather paths store
 // theta_out; the FP64, Pfaffian and two-chain paths do not.
 bool sampler_writes_theta(const MachineDev& m, int fp64, const SamplerShape& sh) {
-    return !fp64 && m.pf.n == 0 && !sh.plan.pair && (sh.plan.use_u || sh.plan.gather);
+    return !fp64 && m.pf.n == 0 && !sh.plan.pair && (sh.plan.screen || sh.plan.use_u || sh.plan.gather);
 }
 
 cudaError_t launch_sampler(const SamplerArgs& a0, int fp64, const SamplerShape& sh, cudaStream_t st) {
     SamplerArgs a = a0;
     a.plan = sh.plan;
+    if (sh.plan.screen) return launch_screen(a, fp64, sh, st);
     const int E = elements_per_lane(a.m.T);
     const void* fn = pick_sampler(E, fp64, sh.plan.use_u, a.m.pf.n > 0, sh.plan.gather, sh.plan.pair);
     if (!fn) return cudaErrorInvalidValue;

@@ -23,6 +23,9 @@ struct MachineDev {
     int symmetric;
     const double2* W64;    // [n][nh] site-major: W64[i*nh + k] = W(i, k)
     const float2* W32;     // FP32 copy of W64
+    // exp(4 W) (first n rows) and exp(-4 W) in FP32, site-major: entries in
+    // pairs (two real parts, two imaginary parts) when nh is even; null: not built
+    const float* P32;
     const double2* hb;     // [nh]
     const double2* vb;     // [n_vb]
     const uint8_t* perm;   // [n][S] perm[f*S + s] = P_s(f)      (symmetric)
@@ -54,6 +57,9 @@ struct SmemPlan {
     int lane_rows;  // gather path, symmetric, nh | 32, T = 32 E (E >= 4): the symmetry
                     // table in lane order (one E-byte load gives a lane its rows)
     int pair;   // table path with two chains per warp
+    int screen;       // FP32 sweep screened by products (sampler_screen.cu)
+    int lane_entries; // entries per lane of the exact sums (elements_per_lane)
+    int p_budget;     // screen: shared-memory bytes that a basic machine's p table may take
     int ham;    // evaluation: bytes of the Hamiltonian tables staged in shared memory (0: read from L2)
 };
 
@@ -205,8 +211,13 @@ struct SamplerShape {
 // 1 asks for two chains per warp where the table path allows it (else, and
 // by default, one chain per warp).
 cudaError_t plan_sampler(const MachineDev& m, int fp64, int n_chains, int n_bonds, SamplerShape* out,
-                         int max_wpb = 0, int pair_mode = -1);
+                         int max_wpb = 0, int pair_mode = -1, bool screen = true);
 cudaError_t launch_sampler(const SamplerArgs& a, int fp64, const SamplerShape& shape, cudaStream_t st);
+// The sweep screened by products (sampler_screen.cu): its plan (false: not for
+// this machine) and its launch.
+bool plan_screen(const MachineDev& m, int fp64, int n_chains, int n_bonds, int max_wpb, SamplerShape* out,
+                 cudaError_t* err);
+cudaError_t launch_screen(const SamplerArgs& a, int fp64, const SamplerShape& sh, cudaStream_t st);
 // The sweeps of several sessions in one launch per entries-per-lane class
 // (a batch): one descriptor per session, its blocks [block0, block0 +
 // blocks) of the launch.

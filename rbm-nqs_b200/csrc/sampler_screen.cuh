@@ -1,0 +1,715 @@
+// sampler_screen.cuh -- FP32 Metropolis sweep (metropolis_sampler.cpp:118-273)
+// whose proposals are screened by products and decided by the ln|cosh| sums
+// only where the screen cannot tell.
+//
+// The decision of a proposal is  0.5 ln u < d,  d = sum_e ln|cosh theta'_e| -
+// sum_e ln|cosh theta_e| + bias, the sums in the fixed order and arithmetic of
+// lnc_sweep_sum on the chain's FP32 theta (decide_exact below: one ex2 and one
+// cosine per entry, for theta and for theta').  The screen computes the same
+// number from z = exp(-2 theta), held in registers: a flip of site f multiplies
+// z by p = exp(4 sigma_f W[P_s(f), k], a table entry, and
+//   ln|cosh theta'| - ln|cosh theta| = ln|1 + z p| - ln|1 + z| - 2 sigma_f Re W,
+// four FMA-pipe operations for the product, three for |1 + z p|^2, one to
+// multiply them up, one lg2 per four entries and no other transcendental.  When
+// |d - 0.5 ln u| exceeds what the two computations can differ by, the screen's
+// decision is the exact one; otherwise (about 1 % of the proposals) theta at the
+// start of the sweep is formed from its configuration in FP64, the sweep's
+// accepted flips are applied to it in FP32, in order, and decide_exact decides.
+// So chains, samples and counters are those of the exact sums, bit for bit.
+//
+// Sessions in FP64 use the same screen; what it cannot tell is decided by the
+// ln|cosh| sums in FP64 (decide_fp64) on theta formed in FP64 from the current
+// configuration: the decisions of the FP64 sweep (sampler.cu run_chain) up to ties
+// of 1e-15.
+//
+// Error bound.  Away from the zeros of cosh both sums are good to a few 1e-5 (512
+// entries).  Near a zero the exact form loses digits: its |1 + w|^2 = 1 + |w|^2 +
+// 2 |w| cos carries the absolute error of the hardware cosine (2^-20.9, growing
+// with the argument) and exponential, so its ln is off by up to 1e-6 / |1 +
+// w|^2 per entry.  The margin is therefore m0 + coef (1 / min |1 + w|^2 at
+// theta' + 1 / min at theta), the minima over the entries, with m0 = 1e-3 + 2e-5
+// max |Re theta| and coef = 2e-6 + 5e-7 max |Im theta|, four times these errors,
+// max over all configurations of the machine (|b| + sum_f |W|).  z is refreshed
+// from theta every kRefresh sweeps: 1000 products of 1.2e-7 each stay below
+// 1e-5.  A machine that can reach |Re theta| > 40 leaves the FP32 range of z:
+// all its proposals take decide_exact.
+//
+// Layout: groups of KB consecutive hidden units with one symmetry index, lane l
+// owns the groups l + 32 j, entries in pairs (packed FP32x2).  Symmetric machines
+// keep p and W of every row in shared memory and find the row of (site, symmetry)
+// in a 16-bit table; basic machines read row f directly, from shared memory or,
+// where p does not fit, from L2.  The loop is bound by issue and latency (ncu, 512
+// entries: 330 warp instructions a proposal, issue 64 % of active cycles, LSU 39 %,
+// FMA pipe 36 %, FP64 2 %; 16 warps at 128 registers: with 20 at 96 the loop
+// spills, 15.8 ms below).  Measured: 16384 chains x 16 sweeps of 128 spins, 512
+// entries, FP32: 19.8 ms by the exact sums, 13.7 screened, 0.12 % of the proposals
+// decided exactly; FP64 sessions, 500 chains x 19 sweeps of 32 spins, 96 entries:
+// 1.32 ms by the sums, 0.22 screened.
+#pragma once
+
+#include "eloc.cuh"
+#include "sweep_common.cuh"
+
+namespace rbmnqs {
+namespace screen {
+
+constexpr int kRefresh = 8;  // sweeps between refreshes of z
+
+// A chain's state between the sweep loop and its services, in the warp's scratch
+// (z and z p of the last proposal: in local memory).  The loop keeps everything
+// in registers and leaves through this state where a proposal needs the exact
+// sums or theta is wanted: what the services use, the loop then neither saves nor
+// shares registers with.
+struct State {
+    uint32_t start[4];  // configuration at the start of the sweep
+    uint32_t sp[4];     // current configuration
+    float LS, lim;      // sum ln|1 + z|, coef / min |1 + z|^2
+    int st, slot, np, applied;
+    uint32_t prop, nacc;
+    uint32_t code;      // the open proposal: sites, bond flag (bit 16), spins (bits 17, 18)
+    float lu, LSn, lim_n;
+    int accept;
+};
+constexpr int kStateBytes = 96;
+static_assert(sizeof(State) <= kStateBytes, "state fits its slot");
+
+// Hidden units per group: as the row loads can be widest for symmetric machines;
+// pairs for basic machines, whose lanes then read consecutive 16 bytes.
+__host__ __device__ inline int group_width(const MachineDev& m) {
+    if (!m.symmetric) return 2;
+    return m.nh % 4 == 0 ? 4 : (m.nh % 2 == 0 ? 2 : 1);
+}
+
+// Shared-memory carve-up, the same arithmetic on host (sizing) and device.
+struct Layout {
+    int p, w, off, row, w64, base, site, bonds, lim, warp0, warp_bytes, total;
+    int qs;    // row stride of p and W in shared memory (bytes)
+    int ws64;  // row stride of the FP64 W (double2), shared or global
+    int p_smem, w64_smem, bonds_smem;
+};
+// p_budget: bytes that the p table of a basic machine may take in shared memory
+__host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, int warps, int p_budget) {
+    Layout L{};
+    const int n = m.n, nh = m.nh, kb = group_width(m);
+    const bool sym = m.symmetric != 0;
+    L.qs = sym ? 4 * eloc::w32_stride(nh, kb, true) : 8 * nh;
+    L.p_smem = sym || 3 * n * L.qs <= p_budget;
+    L.w64_smem = sym && n * nh * 16 <= 32 * 1024;
+    L.ws64 = L.w64_smem ? eloc::w64_stride(nh) : nh;
+    L.bonds_smem = n_bonds * 8 <= 8 * 1024;
+    L.warp_bytes = kStateBytes + eloc::a16(m.T * 8) + eloc::a16(n * 4);
+    int at = 0;
+    auto take = [&](int bytes) {
+        const int o = at;
+        at += eloc::a16(bytes);
+        return o;
+    };
+    // symmetric: two signs of n + 1 rows (row n: zero, read by groups beyond T)
+    L.p = take(L.p_smem ? 2 * (n + 1) * L.qs : 0);
+    L.w = take(L.p_smem ? (n + 1) * L.qs : 0);
+    L.off = take(sym ? 2 * n * (m.S + 1) : 0);
+    L.row = take(sym ? n * (m.S + 1) : 0);
+    L.w64 = take(L.w64_smem ? n * L.ws64 * 16 : 0);
+    L.base = take(m.T * 16);
+    L.site = take((n + 1) * 8);
+    L.bonds = take(L.bonds_smem ? n_bonds * 8 : 0);
+    L.lim = take(8);
+    L.warp0 = at;
+    L.total = at + warps * L.warp_bytes;
+    return L;
+}
+
+__device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsigned char* smem) {
+    const MachineDev& m = a.m;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int n = m.n, nh = m.nh, S = m.S, SP = S + 1;
+    const bool sym = m.symmetric != 0;
+    float* site = reinterpret_cast<float*>(smem + L.site);
+    unsigned* lim = reinterpret_cast<unsigned*>(smem + L.lim);
+    if (L.p_smem) {
+        const int per = L.qs / 8;  // 8-byte slots a row, the padding zero
+        float2* P = reinterpret_cast<float2*>(smem + L.p);
+        float2* W = reinterpret_cast<float2*>(smem + L.w);
+        for (int i = tid; i < 2 * (n + 1) * per; i += nt) {
+            const int sg = i / ((n + 1) * per), r = i / per - sg * (n + 1), k = i % per;
+            P[i] = r < n && k < nh ? reinterpret_cast<const float2*>(m.P32)[(sg * n + r) * nh + k]
+                                   : make_float2(0.f, 0.f);
+        }
+        for (int i = tid; i < (n + 1) * per; i += nt) {
+            const int r = i / per, k = i % per;
+            W[i] = r < n && k < nh ? m.W32[r * nh + k] : make_float2(0.f, 0.f);
+        }
+    }
+    if (sym) {
+        uint16_t* off = reinterpret_cast<uint16_t*>(smem + L.off);
+        uint8_t* row = smem + L.row;
+        for (int i = tid; i < n * SP; i += nt) {
+            const int f = i / SP, s = i - f * SP, r = s < S ? (int)m.perm[f * S + s] : n;
+            off[i] = (uint16_t)(r * L.qs);
+            row[i] = (uint8_t)r;
+        }
+    }
+    if (L.w64_smem) {
+        double2* W = reinterpret_cast<double2*>(smem + L.w64);
+        for (int i = tid; i < n * nh; i += nt) W[i / nh * L.ws64 + i % nh] = m.W64[i];
+    }
+    if (L.bonds_smem) {
+        int2* b = reinterpret_cast<int2*>(smem + L.bonds);
+        for (int i = tid; i < a.n_prop_bonds; i += nt) b[i] = a.prop_bonds[i];
+    }
+    // Re v (bias term of the exact sum) beside sum_e Re W_fe + Re v
+    if (tid < 2) lim[tid] = 0;
+    __syncthreads();
+    const double2* W64 = L.w64_smem ? reinterpret_cast<const double2*>(smem + L.w64) : m.W64;
+    // theta of the all-up configuration, and the bounds |b| + sum_f |W|
+    double2* base = reinterpret_cast<double2*>(smem + L.base);
+    for (int t = tid; t < m.T; t += nt) {
+        const int k = t % nh, s = t / nh;
+        double2 acc = m.hb[k];
+        float bx = fabsf((float)acc.x), by = fabsf((float)acc.y);
+        for (int f = 0; f < n; f++) {
+            const double2 w = W64[(sym ? (int)smem[L.row + f * SP + s] : f) * L.ws64 + k];
+            acc.x += w.x;
+            acc.y += w.y;
+            bx += fabsf((float)w.x);
+            by += fabsf((float)w.y);
+        }
+        base[t] = acc;
+        // non-finite weights give bounds above any limit
+        atomicMax(&lim[0], __float_as_uint(bx == bx ? bx : 1e30f));
+        atomicMax(&lim[1], __float_as_uint(by == by ? by : 1e30f));
+    }
+    for (int f = tid >> 5; f <= n; f += nt >> 5) {  // a warp per site
+        double acc = 0;
+        if (f < n)
+            for (int t = tid & 31; t < m.T; t += 32)
+                acc += W64[(sym ? (int)smem[L.row + f * SP + t / nh] : f) * L.ws64 + t % nh].x;
+        acc = warp_sum(acc);
+        if ((tid & 31) == 0) {
+            const float v = f < n ? (float)m.vb[f % m.n_vb].x : 0.f;
+            site[2 * f] = v;
+            site[2 * f + 1] = f < n ? (float)(acc + m.vb[f % m.n_vb].x) : 0.f;
+        }
+    }
+    __syncthreads();
+}
+
+// A warp's scratch: the configuration at the start of the sweep (16 bytes),
+// theta [T] in FP32, the sweep's accepted flips.
+__device__ __forceinline__ float2* theta_scratch(unsigned char* wscr) { return reinterpret_cast<float2*>(wscr + 16); }
+
+// One chain.  wscr: the warp's scratch (theta [T] FP32, the sweep's accepted
+// flips [n]).  PS: p and W rows in shared memory (always for symmetric machines).
+template <int KB, int NG, bool SYM, bool PS, bool F64>
+__device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L, unsigned char* smem,
+                                          unsigned char* wscr, int chain, int lane) {
+    constexpr int E = KB * NG, NP = E / 2;
+    static_assert(E % 2 == 0 && (SYM ? PS : KB == 2), "entries in pairs; basic machines in groups of two");
+    const MachineDev& m = a.m;
+    const int n = m.n, nh = m.nh, T = m.T, SP = m.S + 1;
+    const uint2 key = make_uint2((uint32_t)a.seed, (uint32_t)(a.seed >> 32));
+    const uint32_t epoch = a.ctl[0];
+    State* S = reinterpret_cast<State*>(wscr);
+    float2* th = reinterpret_cast<float2*>(wscr + kStateBytes);
+    uint32_t* plist = reinterpret_cast<uint32_t*>(wscr + kStateBytes + eloc::a16(T * 8));
+    {
+        uint32_t sp[4];
+        chain_start(a, chain, key, epoch, sp);
+        if (lane < 4) S->sp[lane] = spin_word(sp, lane);
+        if (lane == 0) {
+            S->st = S->np = S->slot = 0;
+            S->prop = prop_base(a);
+            S->nacc = 0;
+        }
+        __syncwarp();
+    }
+    const double2* base = reinterpret_cast<const double2*>(smem + L.base);
+    const double2* W64 = L.w64_smem ? reinterpret_cast<const double2*>(smem + L.w64) : m.W64;
+    const uint8_t* rows = smem + L.row;
+    const uint32_t wa = smem_addr(smem + L.w);
+    const uint32_t sa = smem_addr(smem + L.site);
+    const uint32_t pa = smem_addr(smem + L.p), oa = smem_addr(smem + L.off);
+    const uint32_t psign = (uint32_t)((n + 1) * L.qs);
+    const int G = T / KB, NGK = nh / KB;
+    // per group: symmetric, the byte offset of its symmetry index in a row of
+    // the offset table; basic, unused.  ko: byte offset of its first entry in a row
+    uint32_t s2[NG], ko[NG];
+#pragma unroll
+    for (int j = 0; j < NG; j++) {
+        const int g = lane + 32 * j;
+        const bool ok = g < G;
+        s2[j] = 2u * (uint32_t)(SYM ? (ok ? g / NGK : m.S) : 0);
+        ko[j] = 8u * (uint32_t)(SYM ? (ok ? (g % NGK) * KB : 0) : (ok ? g * KB : 0));
+    }
+
+    // theta of configuration S->start (FP64, down spins in increasing order),
+    // rounded to FP32 into the scratch, two groups at a time
+    auto theta_of = [&]() {
+        constexpr int NJ = NG >= 2 ? 2 : 1;
+#pragma unroll 1
+        for (int j0 = 0; j0 < NG; j0 += NJ) {
+            double2 acc[NJ * KB];
+            int gs[NJ], gk[NJ];
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {
+                const int g = min(lane + 32 * (j0 + j), G - 1);  // beyond T: computed, not stored
+                gs[j] = SYM ? g / NGK : 0;
+                gk[j] = SYM ? (g - gs[j] * NGK) * KB : g * KB;
+#pragma unroll
+                for (int i = 0; i < KB; i++) acc[KB * j + i] = base[KB * g + i];
+            }
+#pragma unroll 1
+            for (int wd = 0; wd < 4; wd++) {
+                uint32_t bits = S->start[wd];
+                while (bits) {
+                    const int f = 32 * wd + __ffs(bits) - 1;
+                    bits &= bits - 1;
+#pragma unroll
+                    for (int j = 0; j < NJ; j++) {
+                        const double2* w = W64 + (SYM ? (int)rows[f * SP + gs[j]] : f) * L.ws64 + gk[j];
+#pragma unroll
+                        for (int i = 0; i < KB; i++) {
+                            const double2 v = w[i];
+                            acc[KB * j + i].x = fma(-2.0, v.x, acc[KB * j + i].x);
+                            acc[KB * j + i].y = fma(-2.0, v.y, acc[KB * j + i].y);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {
+                const int g = lane + 32 * (j0 + j);
+                if (g < G)
+#pragma unroll
+                    for (int i = 0; i < KB; i++)
+                        th[KB * g + i] = make_float2((float)acc[KB * j + i].x, (float)acc[KB * j + i].y);
+            }
+        }
+        __syncwarp();
+    };
+    // W entry t of site f
+    auto wrow = [&](int f, int t) -> float2 {
+        if constexpr (SYM) {
+            const int g = t / KB, q = NGK == 1 ? g : g / NGK, k = (g - q * NGK) * KB + t % KB;
+            return lds_f2(wa + (uint32_t)(rows[f * SP + q] * L.qs) + 8u * k);
+        } else if constexpr (PS) {
+            return lds_f2(wa + (uint32_t)(f * L.qs) + 8u * t);
+        } else {
+            return __ldg(m.W32 + f * nh + t);
+        }
+    };
+    // The FP64 sessions' decision: u < |psi'/psi|^2 by the ln|cosh| sums in FP64,
+    // theta formed from the current configuration.
+    auto decide_fp64 = [&](uint32_t code, uint32_t prop) -> bool {
+        const int f0 = code & 255u, f1 = (code >> 8) & 255u;
+        const bool bond = (code >> 16) & 1u;
+        const double g0 = (code >> 17) & 1u ? 2.0 : -2.0, g1 = (code >> 18) & 1u ? 2.0 : -2.0;
+        double d = 0;
+#pragma unroll 1
+        for (int t = lane; t < T; t += 32) {
+            const int q = SYM ? t / nh : 0, k = SYM ? t - q * nh : t;
+            double2 x = base[t];
+#pragma unroll 1
+            for (int wd = 0; wd < 4; wd++) {
+                uint32_t bits = S->sp[wd];
+                while (bits) {
+                    const int f = 32 * wd + __ffs(bits) - 1;
+                    bits &= bits - 1;
+                    const double2 w = W64[(SYM ? (int)rows[f * SP + q] : f) * L.ws64 + k];
+                    x.x = fma(-2.0, w.x, x.x);
+                    x.y = fma(-2.0, w.y, x.y);
+                }
+            }
+            double2 w = W64[(SYM ? (int)rows[f0 * SP + q] : f0) * L.ws64 + k];
+            double2 y = make_double2(fma(g0, w.x, x.x), fma(g0, w.y, x.y));
+            if (bond) {
+                w = W64[(SYM ? (int)rows[f1 * SP + q] : f1) * L.ws64 + k];
+                y = make_double2(fma(g1, w.x, y.x), fma(g1, w.y, y.y));
+            }
+            d += lnc_re<double>(y.x, y.y) - lnc_re<double>(x.x, x.y);
+        }
+        d = warp_sum(d) + g0 * m.vb[f0 % m.n_vb].x;
+        if (bond) d += g1 * m.vb[f1 % m.n_vb].x;
+        const uint4 r = philox4x32(make_uint4(prop, epoch, (uint32_t)chain, 0), key);
+        return unit24<double>(r.z) < exp(2.0 * d);
+    };
+    // d of a proposal (code: sites, bond flag in bit 16, spins of the sites in
+    // bits 17 and 18) by the ln|cosh| sums of theta and theta' over the entries
+    // lane + 32 e, in the arithmetic of lnc_sweep_sum and sweep_sum, after the
+    // accepted flips from `applied` on have been applied to theta in the scratch
+    auto decide_exact = [&](uint32_t code, int applied, int np) -> float {
+#pragma unroll 1
+        for (; applied < np; applied++) {
+            const uint32_t c = plist[applied];
+            const int q0 = c & 255u, q1 = (c >> 8) & 255u;
+            const float h0 = (c >> 17) & 1u ? 2.f : -2.f, h1 = (c >> 18) & 1u ? 2.f : -2.f;
+            const bool two = (c >> 16) & 1u;
+#pragma unroll 4
+            for (int t = lane; t < T; t += 32) {
+                float2 v = __ffma2_rn(make_float2(h0, h0), wrow(q0, t), th[t]);
+                if (two) v = __ffma2_rn(make_float2(h1, h1), wrow(q1, t), v);
+                th[t] = v;
+            }
+        }
+        const int f0 = code & 255u, f1 = (code >> 8) & 255u;
+        const bool bond = (code >> 16) & 1u;
+        const float g0 = (code >> 17) & 1u ? 2.f : -2.f, g1 = (code >> 18) & 1u ? 2.f : -2.f;
+        float sa0 = 0.f, lg0 = 0.f, sa1 = 0.f, lg1 = 0.f;
+#pragma unroll 1
+        for (int e0 = 0; e0 < a.plan.lane_entries; e0 += 4) {
+            float pm0 = 1.f, pm1 = 1.f;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (e0 + q >= a.plan.lane_entries) break;
+                const int t = lane + 32 * (e0 + q);
+                float2 x = make_float2(0.f, 0.f), y = x;
+                if (t < T) {
+                    x = th[t];
+                    y = __ffma2_rn(make_float2(g0, g0), wrow(f0, t), x);
+                    if (bond) y = __ffma2_rn(make_float2(g1, g1), wrow(f1, t), y);
+                }
+                const float ax = fabsf(x.x), ay = fabsf(y.x);
+                const float zx = ex2_ftz(ax * -2.88539008177792681f), zy = ex2_ftz(ay * -2.88539008177792681f);
+                const float cx = cos_ftz(2.f * x.y), cy = cos_ftz(2.f * y.y);
+                pm0 *= fmaf(zx, fmaf(2.f, cx, zx), 1.f);
+                pm1 *= fmaf(zy, fmaf(2.f, cy, zy), 1.f);
+                sa0 += ax;
+                sa1 += ay;
+            }
+            lg0 += lg2_ftz(pm0);
+            lg1 += lg2_ftz(pm1);
+        }
+        const float s0 = fmaf(0.346573590279972655f, lg0, sa0), s1 = fmaf(0.346573590279972655f, lg1, sa1);
+        float d = sweep_sum(s1 - s0);
+        d = fmaf(g0, lds_f2(sa + 8u * f0).x, d);
+        return fmaf(g1, lds_f2(sa + 8u * f1).x, d);
+    };
+
+    // squared moduli of 1 + z over the lane's entries: the sum of their lg2 in
+    // 2^-16 steps over the warp (times ln 2 / 2: sum ln|1 + z|) and their minimum
+    auto log_sum = [&](const float2 (&xr)[NP], const float2 (&xi)[NP], float& mn) -> float {
+        float lg = 0.f, lo = 1e30f;
+        const float2 one = make_float2(1.f, 1.f);
+#pragma unroll
+        for (int p = 0; p < NP; p += 2) {
+            const float2 u = __fadd2_rn(xr[p], one);
+            float2 q = __ffma2_rn(u, u, __fmul2_rn(xi[p], xi[p]));
+            lo = fminf(lo, fminf(q.x, q.y));
+            if (p + 1 < NP) {
+                const float2 v = __fadd2_rn(xr[p + 1], one);
+                const float2 r = __ffma2_rn(v, v, __fmul2_rn(xi[p + 1], xi[p + 1]));
+                lo = fminf(lo, fminf(r.x, r.y));
+                q = __fmul2_rn(q, r);
+            }
+            lg += lg2_ftz(q.x * q.y);
+        }
+        // out of range (or NaN): a minimum of 0, an infinite margin
+        mn = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(fabsf(lg) < 1000.f ? lo : 0.f)));
+        return (float)__reduce_add_sync(kFull, __float2int_rn(lg * 65536.f)) * (0.346573590279972655f / 65536.f);
+    };
+    const float bre = __uint_as_float(reinterpret_cast<const unsigned*>(smem + L.lim)[0]);
+    const float bim = __uint_as_float(reinterpret_cast<const unsigned*>(smem + L.lim)[1]);
+    const float m0 = bre > 40.f ? __int_as_float(0x7f800000) : 1e-3f + 2e-5f * bre;
+    const float coef = 2e-6f + 5e-7f * bim;
+    // w = x p(f, spin sg)
+    auto times_p = [&](int f, int sg, const float2 (&xr)[NP], const float2 (&xi)[NP], float2 (&wr)[NP],
+                       float2 (&wi)[NP]) {
+        auto mul = [&](int p, float2 pr, float2 pi) {
+            const float2 yr = xr[p], yi = xi[p];
+            wr[p] = __ffma2_rn(yr, pr, __fmul2_rn(make_float2(-yi.x, -yi.y), pi));
+            wi[p] = __ffma2_rn(yr, pi, __fmul2_rn(yi, pr));
+        };
+        if constexpr (PS) {
+            const uint32_t pb = pa + (sg ? psign : 0u) + (SYM ? 0u : (uint32_t)(f * L.qs));
+            const uint32_t ob = oa + 2u * (uint32_t)(f * SP);
+            if constexpr (KB == 4) {
+#pragma unroll
+                for (int j = 0; j < NG; j++) {
+                    const uint32_t at = pb + eloc::lds16(ob + s2[j]) + ko[j];
+                    const float4 v0 = eloc::lds128(at), v1 = eloc::lds128(at + 16);
+                    mul(2 * j, make_float2(v0.x, v0.y), make_float2(v0.z, v0.w));
+                    mul(2 * j + 1, make_float2(v1.x, v1.y), make_float2(v1.z, v1.w));
+                }
+            } else if constexpr (KB == 2) {
+#pragma unroll
+                for (int j = 0; j < NG; j++) {
+                    const float4 v = eloc::lds128(pb + (SYM ? eloc::lds16(ob + s2[j]) : 0u) + ko[j]);
+                    mul(j, make_float2(v.x, v.y), make_float2(v.z, v.w));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < NG; j += 2) {
+                    const float2 v0 = eloc::lds64(pb + eloc::lds16(ob + s2[j]) + ko[j]);
+                    const float2 v1 = eloc::lds64(pb + eloc::lds16(ob + s2[j + 1]) + ko[j + 1]);
+                    mul(j / 2, make_float2(v0.x, v1.x), make_float2(v0.y, v1.y));
+                }
+            }
+        } else {
+            const char* pb = reinterpret_cast<const char*>(m.P32) + (size_t)(sg * n + f) * (8 * nh);
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(pb + ko[j]));
+                mul(j, make_float2(v.x, v.y), make_float2(v.z, v.w));
+            }
+        }
+    };
+
+    const int2* bonds = L.bonds_smem ? reinterpret_cast<const int2*>(smem + L.bonds) : a.prop_bonds;
+    const int total = segment_sweeps(a);
+    const uint32_t thr = a.bond_thr24;
+    volatile float hold[8 * NP];  // z, then z p of the open proposal
+    bool open = false;            // the loop left at a proposal that needs the exact sums
+    for (;;) {
+        if (!open) {
+            // the start of sweep st with theta wanted: z from theta, or theta
+            // of the final configuration
+            const int st = S->st;
+            if (lane < 4) S->start[lane] = S->sp[lane];
+            __syncwarp();
+            if (st == 0 && a.theta_in && a.plan.lane_rows) {
+                const float2* src = a.theta_in + (size_t)chain * 32 * a.plan.lane_entries;
+                for (int t = lane; t < T; t += 32) th[t] = src[t];
+                __syncwarp();
+            } else {
+                theta_of();
+            }
+            if (st == total) break;
+            float2 zr[NP], zi[NP];
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int g = lane + 32 * j;
+#pragma unroll
+                for (int i = 0; i < KB; i++) {
+                    float2 z = make_float2(0.f, 0.f);
+                    if (g < G) {
+                        const float2 t = th[KB * g + i];
+                        const float r = ex2_ftz(t.x * -2.88539008177792681f);
+                        float s, c;
+                        sincos_r(2.f * t.y, &s, &c);
+                        z = make_float2(r * c, -r * s);
+                    }
+                    const int e = j * KB + i;
+                    if (e & 1) {
+                        zr[e >> 1].y = z.x;
+                        zi[e >> 1].y = z.y;
+                    } else {
+                        zr[e >> 1].x = z.x;
+                        zi[e >> 1].x = z.y;
+                    }
+                }
+            }
+            float mn;
+            const float ls = log_sum(zr, zi, mn);
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                hold[4 * p] = zr[p].x;
+                hold[4 * p + 1] = zr[p].y;
+                hold[4 * p + 2] = zi[p].x;
+                hold[4 * p + 3] = zi[p].y;
+            }
+            if (lane == 0) {
+                S->LS = ls;
+                S->lim = __fdividef(coef, mn);
+                S->applied = 0;
+                S->accept = 0;
+            }
+            __syncwarp();
+        } else {
+            const int np = S->np;
+            bool accept;
+            if constexpr (F64) {
+                accept = decide_fp64(S->code, S->prop - 1);
+            } else {
+                int applied = S->applied;
+                if (applied < 0) {
+                    theta_of();
+                    applied = 0;
+                }
+                accept = S->lu < decide_exact(S->code, applied, np);
+            }
+            __syncwarp();
+            if (lane == 0) {
+                S->applied = np;
+                S->accept = accept;
+                if (accept) {
+                    const uint32_t c = S->code;
+                    S->LS = S->LSn;
+                    S->lim = S->lim_n;
+                    if constexpr (!F64) plist[np] = c;
+                    S->np = np + 1;
+                    S->nacc++;
+                    S->sp[(c & 255u) >> 5] ^= 1u << (c & 31u);
+                    if ((c >> 16) & 1u) S->sp[((c >> 8) & 255u) >> 5] ^= 1u << ((c >> 8) & 31u);
+                }
+            }
+            __syncwarp();
+        }
+        // ---- the sweep loop, from the state
+        float2 zr[NP], zi[NP];
+        {
+            const int o = S->accept ? 4 * NP : 0;
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                zr[p] = make_float2(hold[o + 4 * p], hold[o + 4 * p + 1]);
+                zi[p] = make_float2(hold[o + 4 * p + 2], hold[o + 4 * p + 3]);
+            }
+        }
+        const uint32_t spa = smem_addr(S->sp);  // the configuration stays in the scratch
+        float LS = S->LS, lim_cur = S->lim;
+        int st = S->st, slot = S->slot, np = S->np, applied = S->applied;
+        uint32_t prop = S->prop, nacc = S->nacc, pcode = 0;
+        float plu = 0.f;
+        auto draw = [&]() {  // this lane's proposal of the batch of 32
+            const uint4 r = philox4x32(make_uint4((prop & ~31u) + lane, epoch, (uint32_t)chain, 0), key);
+            uint32_t f0, f1, bond;
+            if ((r.x >> 8) < thr) {
+                const int2 b = bonds[pick(r.y, (uint32_t)a.n_prop_bonds)];
+                f0 = (uint32_t)b.x;
+                f1 = (uint32_t)b.y;
+                bond = 1;
+            } else {
+                f0 = pick(r.y, (uint32_t)n);
+                f1 = (uint32_t)n;
+                bond = 0;
+            }
+            pcode = f0 | (f1 << 8) | (bond << 16);
+            plu = 0.346573590279972655f * lg2_ftz(unit24<float>(r.z));  // 0.5 ln u
+        };
+        if (prop & 31u) draw();
+        open = false;
+        for (;;) {
+            if (slot >= n) {  // the sweep is done
+                if (const int j = sample_slot(a, st); j >= 0) {
+                    const size_t idx = (size_t)chain * a.spc + j;
+                    __syncwarp();
+                    if (lane < 4) a.samples[4 * idx + lane] = S->sp[lane];
+                }
+                st++;
+                slot = np = 0;
+                applied = -1;
+                if (st == total || st % kRefresh == 0) break;
+                if (lane < 4) S->start[lane] = S->sp[lane];
+            }
+            if ((prop & 31u) == 0) draw();
+            const int src = prop & 31u;
+            const uint32_t code = __shfl_sync(kFull, pcode, src);
+            const float lu = __shfl_sync(kFull, plu, src);
+            prop++;
+            const int f0 = code & 255u, f1 = (code >> 8) & 255u;
+            const bool bond = (code >> 16) != 0;
+            slot += bond ? 2 : 1;
+            const uint32_t b0 = (lds_u32(spa + ((f0 >> 5) << 2)) >> (f0 & 31)) & 1u;
+            const uint32_t b1 = bond ? (lds_u32(spa + ((f1 >> 5) << 2)) >> (f1 & 31)) & 1u : 0u;
+            const float g0 = b0 ? 2.f : -2.f;  // -2 sigma_f
+            const float g1 = b1 ? 2.f : -2.f;
+            float2 wr[NP], wi[NP];
+            times_p(f0, b0, zr, zi, wr, wi);
+            if (bond) times_p(f1, b1, wr, wi, wr, wi);
+            float mn;
+            const float LSn = log_sum(wr, wi, mn);
+            const float lim_new = __fdividef(coef, mn);
+            const float D = fmaf(g1, lds_f2(sa + 8u * f1).y, fmaf(g0, lds_f2(sa + 8u * f0).y, LSn - LS));
+            const uint32_t full = code | (b0 << 17) | (b1 << 18);
+            if (!(fabsf(D - lu) > m0 + lim_new + lim_cur)) {
+#pragma unroll
+                for (int p = 0; p < NP; p++) {
+                    hold[4 * (NP + p)] = wr[p].x;
+                    hold[4 * (NP + p) + 1] = wr[p].y;
+                    hold[4 * (NP + p) + 2] = wi[p].x;
+                    hold[4 * (NP + p) + 3] = wi[p].y;
+                }
+                if (lane == 0) {
+                    S->code = full;
+                    S->lu = lu;
+                    S->LSn = LSn;
+                    S->lim_n = lim_new;
+                }
+                open = true;
+                break;
+            }
+            if (lu < D) {
+#pragma unroll
+                for (int p = 0; p < NP; p++) {
+                    zr[p] = wr[p];
+                    zi[p] = wi[p];
+                }
+                LS = LSn;
+                lim_cur = lim_new;
+                if (lane == 0) {
+                    if constexpr (!F64) plist[np] = full;
+                    S->sp[f0 >> 5] ^= 1u << (f0 & 31);
+                    if (bond) S->sp[f1 >> 5] ^= 1u << (f1 & 31);
+                }
+                __syncwarp();
+                np++;
+                nacc++;
+            }
+        }
+        // ---- back to the state
+        if (open) {
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                hold[4 * p] = zr[p].x;
+                hold[4 * p + 1] = zr[p].y;
+                hold[4 * p + 2] = zi[p].x;
+                hold[4 * p + 3] = zi[p].y;
+            }
+        }
+        if (lane == 0) {
+            S->LS = LS;
+            S->lim = lim_cur;
+            S->st = st;
+            S->slot = slot;
+            S->np = np;
+            S->applied = applied;
+            S->prop = prop;
+            S->nacc = nacc;
+        }
+        __syncwarp();
+        if (!open && st == total && !a.theta_out) break;
+    }
+    if (a.theta_out) {
+        // FP32 theta of the final configuration, zero beyond T
+        const int TP = 32 * a.plan.lane_entries;
+        float2* dst = a.theta_out + (size_t)chain * TP;
+        for (int t = lane; t < TP; t += 32) dst[t] = t < T ? th[t] : make_float2(0.f, 0.f);
+    }
+    const uint32_t sp[4] = {S->sp[0], S->sp[1], S->sp[2], S->sp[3]};
+    chain_finish(a, chain, lane, sp, S->nacc, S->prop);
+    __syncwarp();
+}
+
+// Threads per block by entries per lane: z and z p of the entries in registers
+// (16 entries: 128 registers; with 640 threads and 96 the loop spills).
+__host__ __device__ constexpr int max_threads(int E) { return E >= 16 ? 512 : (E >= 8 ? 768 : 896); }
+
+template <int KB, int NG, bool SYM, bool PS, bool F64>
+__global__ void __launch_bounds__(max_threads(KB* NG), 1) screen_kernel(const SamplerArgs a, const Layout L) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    load_tables(a, L, smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int total_warps = (blockDim.x >> 5) * gridDim.x;
+    // consecutive chains on different SMs
+    for (int chain = warp * gridDim.x + blockIdx.x; chain < a.n_chains; chain += total_warps)
+        run_chain<KB, NG, SYM, PS, F64>(a, L, smem, smem + L.warp0 + warp * L.warp_bytes, chain, lane);
+}
+
+template <int KB, int NG, bool SYM, bool PS, bool F64> const void* fn() {
+    return reinterpret_cast<const void*>(screen_kernel<KB, NG, SYM, PS, F64>);
+}
+
+// groups per lane
+inline int groups(const MachineDev& m) {
+    const int kb = group_width(m), G = m.T / kb;
+    int ng = kb == 1 ? 2 : 1;  // entries come in pairs
+    while (32 * ng < G) ng *= 2;
+    return ng;
+}
+
+// kernel of a machine; the instantiations are split over two files that compile
+// in parallel (null: none)
+const void* pick_fp32(const MachineDev& m, bool p_smem);
+const void* pick_fp64(const MachineDev& m, bool p_smem);
+
+}  // namespace screen
+}  // namespace rbmnqs

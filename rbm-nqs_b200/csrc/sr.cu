@@ -1030,7 +1030,7 @@ cudaError_t launch_heun_finish(double2* params, double2* x, int P, const Schedul
 
 // Parameter vector -> kernel layouts (site-major W in FP64 and FP32).
 __global__ void unpack_weights(const double2* params, int n, int n_vb, int nh, double2* vb, double2* hb, double2* W64,
-                               float2* W32) {
+                               float2* W32, float* P32) {
     const int tot = n * nh;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < tot + nh + n_vb; i += gridDim.x * blockDim.x) {
         if (i < n_vb) {
@@ -1043,6 +1043,18 @@ __global__ void unpack_weights(const double2* params, int n, int n_vb, int nh, d
             const double2 w = params[i];
             W64[j * nh + k] = w;
             W32[j * nh + k] = make_float2((float)w.x, (float)w.y);
+            if (P32) {  // exp(+-4 W), entry k of row j (MachineDev::P32)
+                double sn, cs;
+                sincos(4.0 * w.y, &sn, &cs);
+                const double g = exp(4.0 * w.x), gi = exp(-4.0 * w.x);
+                const int at = (nh & 1) ? 2 * k : 4 * (k >> 1) + (k & 1), im = (nh & 1) ? 1 : 2;
+                float* up = P32 + 2 * (size_t)j * nh + at;
+                float* dn = up + 2 * (size_t)n * nh;
+                up[0] = (float)(g * cs);
+                up[im] = (float)(g * sn);
+                dn[0] = (float)(gi * cs);
+                dn[im] = (float)(-gi * sn);
+            }
         }
     }
 }
@@ -1182,8 +1194,8 @@ cudaError_t launch_sgd_direction(const double2* F, double2* x, int P, double rea
 }
 
 cudaError_t launch_unpack(const double2* params, int n, int n_vb, int nh, double2* vb, double2* hb, double2* W64,
-                          float2* W32, cudaStream_t st) {
-    unpack_weights<<<148, 256, 0, st>>>(params, n, n_vb, nh, vb, hb, W64, W32);
+                          float2* W32, float* P32, cudaStream_t st) {
+    unpack_weights<<<148, 256, 0, st>>>(params, n, n_vb, nh, vb, hb, W64, W32, P32);
     return cudaGetLastError();
 }
 

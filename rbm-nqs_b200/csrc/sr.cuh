@@ -278,6 +278,6 @@ cudaError_t launch_cg_mfree(const void* O, int fp64, const double2* d, double no
                             const ScheduleDev* sch, double r1, double r2, double rd, int max_it, double rtol,
                             const MfreePlan& pl, const MfreeWork& w, CgResultDev* res, cudaStream_t st);
 cudaError_t launch_unpack(const double2* params, int n, int n_vb, int nh, double2* vb, double2* hb, double2* W64,
-                          float2* W32, cudaStream_t st);
+                          float2* W32, float* P32, cudaStream_t st);
 
 }  // namespace rbmnqs

@@ -11,6 +11,7 @@
 // until the process exits.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -20,10 +21,12 @@
 namespace {
 
 constexpr int kMaxP = RBMNQS_NOALLOC_MAX_PARAMS;
-constexpr int kSplits = 2;  // sample-range splits of the Gram accumulation
 constexpr size_t kMat = (size_t)kMaxP * kMaxP * sizeof(double2);
-// partial Gram sums [kSplits][P][P] | Gram G [P][P] | S_reg [P][P] | CG status
-constexpr size_t kScratchBytes = (kSplits + 2) * kMat + 256;
+// partial Gram sums [splits][P][P] | Gram G [P][P] | S_reg [P][P], and the CG
+// status in the last 256 bytes.  The sample-range splits fill what the matrices
+// leave: two at kMaxP parameters, more below, up to a Gram launch that fills the
+// GPU (133 parameters, 4096 samples: 2 splits 280 us, 12 splits 137 us).
+constexpr size_t kScratchBytes = 4 * kMat + 256;
 
 // The scratch array.  In host code this name is only a host-side stand-in:
 // the device address comes from cudaGetSymbolAddress, once per device.
@@ -72,16 +75,16 @@ extern "C" int rbmnqs_sr_solve_noalloc(const double* O, int32_t N, int32_t P, in
     }
     const size_t mat = (size_t)P * P * sizeof(double2);
     double2* part = reinterpret_cast<double2*>(base);
-    double2* G = reinterpret_cast<double2*>(base + kSplits * mat);
-    double2* Sreg = reinterpret_cast<double2*>(base + (kSplits + 1) * mat);
-    auto* res = reinterpret_cast<rbmnqs::CgResultDev*>(base + (kSplits + 2) * mat);
+    const int room = (int)(4 * kMat / mat) - 2;
+    const int splits = std::min(rbmnqs::gram_splits(N, P), room);
+    double2* G = reinterpret_cast<double2*>(base + splits * mat);
+    double2* Sreg = reinterpret_cast<double2*>(base + (splits + 1) * mat);
+    auto* res = reinterpret_cast<rbmnqs::CgResultDev*>(base + 4 * kMat);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // the array keeps the previous call's contents: the CG status is the only
     // part read before being written
     e = cudaMemsetAsync(res, 0, sizeof(*res), st);
     if (e != cudaSuccess) return fail(RBMNQS_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    int splits = kSplits;
-    if (N < 16 * splits) splits = 1;
     const auto* O2 = reinterpret_cast<const double2*>(O);
     if ((e = rbmnqs::launch_gram_fp64(O2, 1, nullptr, N, P, splits, part, G, st)) != cudaSuccess ||
         (e = rbmnqs::launch_solve_prep(G, N, norm, reinterpret_cast<const double2*>(d), diag, P, n_neural, r1, r2,

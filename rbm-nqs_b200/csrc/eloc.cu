@@ -46,7 +46,6 @@ cudaError_t launch_eloc_fast(const EvalArgs& a, cudaStream_t st) {
     const MachineDev& m = a.m;
     if (m.pf.n > 0 || !a.tt.terms || a.ratio || a.tt.nf_max > 6 || m.n > 255) return cudaErrorNotSupported;
     if (a.B == 0) return cudaSuccess;
-    if (const cudaError_t es = launch_eloc_sym(a, st); es != cudaErrorNotSupported) return es;
     const int kb = m.nh % 4 == 0 ? 4 : (m.nh % 2 == 0 ? 2 : 1);
     const int G = m.T / kb;
     int ng = kb == 1 ? 2 : 1;  // entries come in pairs

@@ -1,6 +1,7 @@
-// eloc_sym.cu -- local energy and log-derivatives of symmetric machines in
-// FP32 (local_op.cpp:31-60, rbm_base.cpp:194-217, rbm_symmetry.cpp:97-130), one
+// eloc_sym.cu -- local energy, log-derivatives and log psi of symmetric machines
+// in FP32 (local_op.cpp:31-60, rbm_base.cpp:194-217, rbm_symmetry.cpp:97-147), one
 // warp per configuration, psi ratios as products without transcendentals.
+// log psi is summed in FP64 from the terms of tanh theta.
 //
 // With z = exp(-2 theta) and delta = -2 sum_f sigma_f W[P_s(f), k] over a term's
 // flips, cosh(theta + delta) / cosh(theta) = exp(-delta) (z + q) / (1 + z),
@@ -253,7 +254,9 @@ __device__ __forceinline__ void reduce_products(int (&e)[KT], float2 (&u)[KT], i
     U = v;
 }
 
-template <int KB, int NG>
+// LP: log psi as well (its FP64 sums cost the kernel without them 9 % when they
+// are compiled into it).
+template <int KB, int NG, bool LP>
 __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* NG))
     eloc_sym_kernel(const EvalArgs a, const SymLayout L) {
     constexpr int E = KB * NG, NP = E / 2;
@@ -384,6 +387,7 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
         // pairs, and the lane's product of 1 + z
         float2 zr[NP], zi[NP];
         double2 D = make_double2(1, 0);
+        double lre = 0, lim = 0;  // sum ln cosh theta (principal values), ln 2 per entry left out
 #pragma unroll
         for (int j = 0; j < NG; j++) {
             double2 acc[KB];
@@ -419,8 +423,13 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                     const double omz = -expm1(-2.0 * aa), w = 1.0 - omz;
                     double s, c;
                     sincos(acc[i].y, &s, &c);
+                    const double X = (1.0 + w) * c, Y = omz * s;
+                    if constexpr (LP) {
+                        lre += aa + 0.5 * log(X * X + Y * Y);
+                        lim += atan2(copysign(omz, x) * s, X);
+                    }
                     if (a.O) {
-                        const double X = (1.0 + w) * c, Y = omz * s, inv = 1.0 / (X * X + Y * Y);
+                        const double inv = 1.0 / (X * X + Y * Y);
                         tn[t0 + i] = make_float2((float)(copysign(omz * (1.0 + w), x) * inv),
                                                  (float)(4.0 * w * s * c * inv));
                     }
@@ -442,6 +451,19 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
             }
         }
 
+        if constexpr (LP) {
+            lre = warp_sum(lre);
+            lim = warp_sum(lim);
+            double bx = 0, by = 0;
+            for (int q = 0; q < n_vb; q++) {
+                double acc = 0;
+                for (int s = lane; s < S; s += 32) acc += sbit(sp, m.orbit[q * S + s]) ? -1.0 : 1.0;
+                acc = warp_sum(acc);
+                bx += sVb[q].x * acc;
+                by += sVb[q].y * acc;
+            }
+            if (lane == 0) a.logpsi[b] = make_double2(bx + lre - 0.69314718055994531 * T, by + lim);
+        }
         if (a.eloc) {
             double ex = 0.0, ey = 0.0;
             // C = prod 1 / (1 + z) = C 2^ec
@@ -567,21 +589,23 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
     }
 }
 
-template <int KB, int NG> const void* fn() { return reinterpret_cast<const void*>(eloc_sym_kernel<KB, NG>); }
+template <int KB, int NG, bool LP> const void* fn() {
+    return reinterpret_cast<const void*>(eloc_sym_kernel<KB, NG, LP>);
+}
 
-const void* pick_sym(int kb, int ng) {
+template <bool LP> const void* pick_sym(int kb, int ng) {
     switch (100 * kb + ng) {
-        case 401: return fn<4, 1>();
-        case 402: return fn<4, 2>();
-        case 404: return fn<4, 4>();
-        case 201: return fn<2, 1>();
-        case 202: return fn<2, 2>();
-        case 204: return fn<2, 4>();
-        case 208: return fn<2, 8>();
-        case 102: return fn<1, 2>();
-        case 104: return fn<1, 4>();
-        case 108: return fn<1, 8>();
-        case 116: return fn<1, 16>();
+        case 401: return fn<4, 1, LP>();
+        case 402: return fn<4, 2, LP>();
+        case 404: return fn<4, 4, LP>();
+        case 201: return fn<2, 1, LP>();
+        case 202: return fn<2, 2, LP>();
+        case 204: return fn<2, 4, LP>();
+        case 208: return fn<2, 8, LP>();
+        case 102: return fn<1, 2, LP>();
+        case 104: return fn<1, 4, LP>();
+        case 108: return fn<1, 8, LP>();
+        case 116: return fn<1, 16, LP>();
     }
     return nullptr;
 }
@@ -598,7 +622,7 @@ cudaError_t launch_eloc_sym(const EvalArgs& a, cudaStream_t st) {
     const int G = m.T / kb;
     int ng = kb == 1 ? 2 : 1;  // entries come in pairs
     while (32 * ng < G) ng *= 2;
-    const void* f = pick_sym(kb, ng);
+    const void* f = a.logpsi ? pick_sym<true>(kb, ng) : pick_sym<false>(kb, ng);
     if (!f) return cudaErrorNotSupported;
     int dev = 0, budget = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);

@@ -2329,9 +2329,15 @@ static cudaError_t launch_eval_warp(const EvalArgs& a, int fp64, int wpb, cudaSt
     RBMNQS_DISPATCH(launch_e, a)
 }
 
-// FP32 E_loc and O_k go to the term-table kernel (eloc.cu) when it supports
-// the machine; log psi, ratios, FP64 and the Pfaffian factor to eval_kernel.
+// FP32 E_loc, O_k and log psi of symmetric machines go to the product kernel
+// (eloc_sym.cu), E_loc and O_k of the others to the term-table kernel (eloc.cu) when
+// it supports the machine; ratios, FP64, the Pfaffian factor and the other log
+// psi to eval_kernel.
 cudaError_t launch_eval(const EvalArgs& a, int fp64, int wpb, cudaStream_t st) {
+    if (!fp64 && !a.ratio && a.tt.terms && a.m.pf.n == 0) {
+        const cudaError_t es = a.B == 0 ? cudaSuccess : launch_eloc_sym(a, st);
+        if (es != cudaErrorNotSupported) return es;
+    }
     if (!fp64 && (a.eloc || a.O) && !a.ratio && a.tt.terms && a.m.pf.n == 0) {
         EvalArgs f = a;
         f.logpsi = nullptr;

@@ -244,8 +244,8 @@ cudaError_t launch_eval(const EvalArgs& a, int fp64, int warps_per_block, cudaSt
 cudaError_t launch_eloc_fast(const EvalArgs& a, cudaStream_t st);
 // The same for symmetric machines, psi ratios as products over tables of the
 // distinct flipped row tuples (eloc_sym.cu); cudaErrorNotSupported when the
-// machine is not symmetric or its tables do not fit, launch_eloc_fast then
-// runs its general kernel.
+// machine is not symmetric or its tables do not fit, launch_eval then runs the
+// general kernels.
 cudaError_t launch_eloc_sym(const EvalArgs& a, cudaStream_t st);
 int elements_per_lane(int T);
 cudaError_t launch_advance(uint32_t* ctl, int reinit, cudaStream_t st);

@@ -327,6 +327,7 @@ struct rbmnqs_handle {
     DevBuf<double2> eval;
     DevBuf<int2> bonds;
     DevBuf<uint32_t> spins, nacc, nprop, ctl, samples;
+    DevBuf<unsigned char> evalbuf;  // eval_common
     DevBuf<double2> E;
     DevBuf<unsigned char> O;
     DevBuf<double2> pd, pf, pe, d, F, emean, part, Sm, Sreg;
@@ -1733,64 +1734,66 @@ int rbmnqs_set_spins(rbmnqs_handle* h, const uint32_t* spins) {
     });
 }
 
+// Buffers of eval_batch and log_psi_over_psi: one allocation in the handle, kept
+// from call to call up to kEvalKeep bytes (cudaMalloc and cudaFree cost more than
+// a small evaluation) and replaced by one of the call's size above.
+constexpr size_t kEvalKeep = size_t(64) << 20;
+
 static void eval_common(rbmnqs_handle* h, const uint32_t* spins, int B, double* logpsi, double* eloc, double* O,
                         const int32_t* flips, int nflips, double* ratio) {
     require(h && spins && B >= 0, "bad arguments");
     if (B == 0) return;
-    DevBuf<uint32_t> ds;
-    DevBuf<double2> dl, de, dr;
-    DevBuf<unsigned char> dO;
-    DevBuf<int> df;
-    ds.alloc((size_t)B * 4);
-    ck(cudaMemcpyAsync(ds.p, spins, (size_t)B * 16, cudaMemcpyHostToDevice, h->st), "c");
+    if (ratio) require(flips && nflips >= 1 && nflips <= 6, "1..6 flips per configuration");
+    // one block: spins | complex results | flips | O | FP64 copy of an FP32 O
+    const size_t cnt = (size_t)B * h->P, osz = h->osize();
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t o_s = take((size_t)B * 16), o_l = take(logpsi ? (size_t)B * 16 : 0),
+                 o_e = take(eloc ? (size_t)B * 16 : 0), o_r = take(ratio ? (size_t)B * 16 : 0),
+                 o_f = take(ratio ? (size_t)B * nflips * sizeof(int) : 0), o_O = take(O ? cnt * osz : 0),
+                 o_D = take(O && !h->fp64 ? cnt * sizeof(double2) : 0);
+    DevBuf<unsigned char> own;
+    if (at > kEvalKeep)
+        own.alloc(at);
+    else if (h->evalbuf.n < at)
+        h->evalbuf.alloc(at);
+    unsigned char* base = at > kEvalKeep ? own.p : h->evalbuf.p;
+    ck(cudaMemcpyAsync(base + o_s, spins, (size_t)B * 16, cudaMemcpyHostToDevice, h->st), "c");
     rbmnqs::EvalArgs a{};
     a.m = h->machine();
     a.H = h->ham();
     a.md = h->mdev.p;
     a.hd = h->hdev.p;
-    a.spins = ds.p;
+    a.spins = reinterpret_cast<const uint32_t*>(base + o_s);
     a.B = B;
     a.plan = rbmnqs::SmemPlan{0, h->w_in_smem, 0, 0, 0};
     a.tt = h->terms.tt;
     a.wrank = h->wrank.p;
-    if (logpsi) {
-        dl.alloc(B);
-        a.logpsi = dl.p;
-    }
-    if (eloc) {
-        de.alloc(B);
-        a.eloc = de.p;
-    }
-    if (O) {
-        dO.alloc((size_t)B * h->P * h->osize());
-        a.O = dO.p;
-    }
+    if (logpsi) a.logpsi = reinterpret_cast<double2*>(base + o_l);
+    if (eloc) a.eloc = reinterpret_cast<double2*>(base + o_e);
+    if (O) a.O = base + o_O;
     if (ratio) {
-        require(flips && nflips >= 1 && nflips <= 6, "1..6 flips per configuration");
-        df.alloc((size_t)B * nflips);
-        dr.alloc(B);
-        ck(cudaMemcpyAsync(df.p, flips, (size_t)B * nflips * sizeof(int), cudaMemcpyHostToDevice, h->st), "c");
-        a.flips = df.p;
+        ck(cudaMemcpyAsync(base + o_f, flips, (size_t)B * nflips * sizeof(int), cudaMemcpyHostToDevice, h->st), "c");
+        a.flips = reinterpret_cast<const int*>(base + o_f);
         a.n_flips = nflips;
-        a.ratio = dr.p;
+        a.ratio = reinterpret_cast<double2*>(base + o_r);
     }
     ck(rbmnqs::launch_eval(a, h->fp64, h->wpb, h->st), "eval kernel");
-    if (logpsi) ck(cudaMemcpyAsync(logpsi, dl.p, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
-    if (eloc) ck(cudaMemcpyAsync(eloc, de.p, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
-    if (ratio) ck(cudaMemcpyAsync(ratio, dr.p, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
+    if (logpsi) ck(cudaMemcpyAsync(logpsi, a.logpsi, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
+    if (eloc) ck(cudaMemcpyAsync(eloc, a.eloc, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
+    if (ratio) ck(cudaMemcpyAsync(ratio, a.ratio, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
     if (O) {
-        const size_t cnt = (size_t)B * h->P;
-        if (h->fp64) {
-            ck(cudaMemcpyAsync(O, dO.p, cnt * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
-        } else {
-            std::vector<float2> tmp(cnt);
-            ck(cudaMemcpyAsync(tmp.data(), dO.p, cnt * sizeof(float2), cudaMemcpyDeviceToHost, h->st), "c");
-            ck(cudaStreamSynchronize(h->st), "sync");
-            for (size_t i = 0; i < cnt; i++) {
-                O[2 * i] = tmp[i].x;
-                O[2 * i + 1] = tmp[i].y;
-            }
+        const void* src = a.O;
+        if (!h->fp64) {  // widened on the device
+            ck(rbmnqs::launch_widen(static_cast<const float2*>(a.O), cnt, reinterpret_cast<double2*>(base + o_D), h->st),
+               "widen");
+            src = base + o_D;
         }
+        ck(cudaMemcpyAsync(O, src, cnt * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
     }
     ck(cudaStreamSynchronize(h->st), "sync");
 }

@@ -625,11 +625,20 @@ __global__ void __launch_bounds__(kThreads) var_diag_kernel(const TO* __restrict
         double s = 0;
         if (q < P) {
             const double2 dq = d[q];
-            for (int n = rg; n < N; n += ngr) {
-                const double2 o = zld(O, (size_t)n * P + q);
+            auto add = [&](double2 o) {
                 const double ex = o.x - dq.x, ey = o.y - dq.y;
                 s = fma(ex, ex, fma(ey, ey, s));
+            };
+            // eight rows' loads in flight before their (ordered) sums
+            int n = rg;
+            for (; n + 7 * ngr < N; n += 8 * ngr) {
+                double2 o[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) o[u] = zld(O, (size_t)(n + u * ngr) * P + q);
+#pragma unroll
+                for (int u = 0; u < 8; u++) add(o[u]);
             }
+            for (; n < N; n += ngr) add(zld(O, (size_t)n * P + q));
         }
         colred[tid] = s;
         __syncthreads();

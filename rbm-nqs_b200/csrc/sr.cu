@@ -57,14 +57,16 @@ __device__ __forceinline__ double2 ld2(const double2* O, size_t i) { return O[i]
 // ------------------------------------------------------------- moments ---
 // Per block over a slice of samples: sum_n O[n][p], sum_n E_n conj(O[n][p]),
 // sum_n E_n (aggregators a_d_, a_dh_, a_h_: aggregator.cpp:190-231), each
-// term weighted by w[n] when w is given (full enumeration, p = |psi|^2).
+// term weighted by w[n] when w is given (full enumeration, p = |psi|^2).  Block
+// (x, y): the samples of slice x, the columns of chunk y.
 template <typename TO>
 __global__ void moments_partial(const TO* O, const double2* E, int N, int P, double2* pd, double2* pf, double2* pe,
                                 const double* w) {
     __shared__ double2 red[32];
     const int nb = gridDim.x;
     const int n0 = (int)((long)N * blockIdx.x / nb), n1 = (int)((long)N * (blockIdx.x + 1) / nb);
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+    const int p = blockIdx.y * blockDim.x + threadIdx.x;
+    if (p < P) {
         double sx = 0, sy = 0, fx = 0, fy = 0;
         auto add = [&](double2 o, int n) {
             if (w) {
@@ -90,6 +92,7 @@ __global__ void moments_partial(const TO* O, const double2* E, int N, int P, dou
         pd[(size_t)blockIdx.x * P + p] = make_double2(sx, sy);
         pf[(size_t)blockIdx.x * P + p] = make_double2(fx, fy);
     }
+    if (blockIdx.y) return;
     double2 es = make_double2(0, 0);
     for (int n = n0 + threadIdx.x; n < n1; n += blockDim.x) {
         const double2 e = E[n];
@@ -647,11 +650,19 @@ __global__ void __launch_bounds__(1024) cg_packed(const double2* A, const double
 // ||r||^2 partial pushed to every CTA, barrier; beta and the whole new p
 // computed by every CTA from its full r and p (the same arithmetic on the
 // same data in every CTA, so the copies agree).  Two cluster barriers per
-// iteration.  The operator, the arithmetic order within a row and the
-// stopping rule are those of cg_packed.
+// iteration.  The operator and the stopping rule are those of cg_packed.
+//
+// An iteration is latency: besides the two cluster barriers one block barrier
+// after the product (half a warp per row) and one after the new p.  Eight warps
+// hold the CTA's rows of x and r in registers and do the same updates and sums,
+// each for the CTA that it writes to, so that no partial crosses the block on
+// its way (133 parameters: 2.5 us per iteration; 2.8 with 256 threads, block
+// sums by two more barriers each and one warp writing to all CTAs).
 constexpr int kClusterCta = 8;
 
-__global__ void __cluster_dims__(kClusterCta, 1, 1) __launch_bounds__(256)
+constexpr int kClusterThreads = 512;
+
+__global__ void __cluster_dims__(kClusterCta, 1, 1) __launch_bounds__(kClusterThreads)
     cg_cluster(const double2* A, const double2* b, double2* xg, int P, int max_it, double rtol, CgResultDev* res) {
     extern __shared__ __align__(16) unsigned char sm[];
     cgx::cluster_group cl = cgx::this_cluster();
@@ -660,88 +671,80 @@ __global__ void __cluster_dims__(kClusterCta, 1, 1) __launch_bounds__(256)
     const int r0 = rank * rp, r1 = min(P, r0 + rp), nr = max(0, r1 - r0);
     double2* Srow = reinterpret_cast<double2*>(sm);  // [rp][P]
     double2* p = Srow + (size_t)rp * P;              // [P] full copy
-    double2* x = p + P;                              // [rp]
-    double2* rf = x + rp;                            // [P] full copy of r
+    double2* rf = p + P;                             // [P] full copy of r
     double2* Ap = rf + P;                            // [rp]
     __shared__ double2 partA[kClusterCta], partB[kClusterCta];
-    __shared__ double2 wred[8];
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-    const int sub = lane & 7;
+    constexpr int NW = kClusterThreads / 32;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5;
     for (int i = tid; i < nr * P; i += nt) Srow[i] = A[(size_t)r0 * P + i];
     for (int i = tid; i < P; i += nt) p[i] = xg[i];
-    for (int i = tid; i < nr; i += nt) x[i] = xg[r0 + i];
-    __syncthreads();
+    cl.sync();  // every CTA runs before its memory is written
 
-    auto cta_sum = [&](double2 v) -> double2 {  // every thread gets the CTA total
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            v.x += __shfl_xor_sync(kFull, v.x, o);
-            v.y += __shfl_xor_sync(kFull, v.y, o);
-        }
-        __syncthreads();
-        if (lane == 0) wred[w] = v;
-        __syncthreads();
-        double2 t = make_double2(0, 0);
-        for (int i = 0; i < nw; i++) {
-            t.x += wred[i].x;
-            t.y += wred[i].y;
-        }
-        return t;
-    };
-    // push this CTA's partial into slot `rank` of every CTA's array
-    auto push = [&](double2* arr, double2 v) {
-        if (tid < kClusterCta) {
-            double2* dst = cl.map_shared_rank(arr, tid);
-            dst[rank] = v;
-        }
-    };
+    // warps 0 .. 7 each hold this CTA's rows of x and r (lane i: rows i and i +
+    // 32), do the same updates, and write to CTA w
+    constexpr int NR = 2;  // rows per lane: at most 64 rows per CTA (cg_cluster_fits: 40)
+    double2 xr[NR], rr[NR];
+    double2* rf_w = cl.map_shared_rank(rf, w % kClusterCta);
+    double2* pa_w = cl.map_shared_rank(partA, w % kClusterCta);
+    double2* pb_w = cl.map_shared_rank(partB, w % kClusterCta);
     auto total = [&](const double2* arr) {
         double2 t = make_double2(0, 0);
+#pragma unroll
         for (int i = 0; i < kClusterCta; i++) {
             t.x += arr[i].x;
             t.y += arr[i].y;
         }
         return t;
     };
-    // local rows of A p; returns this thread's share of p^H Ap
-    auto matvec = [&]() -> double2 {
-        double2 pap = make_double2(0, 0);
-        for (int q0 = 4 * w; q0 < nr; q0 += 4 * nw) {
-            const int q = q0 + (lane >> 3);
-            const bool ok = q < nr;
+    // local rows of A p, half a warp per row
+    auto matvec = [&]() {
+        const int sub = lane & 15;
+        for (int q0 = 2 * w; q0 < nr; q0 += 2 * NW) {
+            const int q = q0 + (lane >> 4);
             double sx = 0, sy = 0;
-            if (ok) {
+            if (q < nr) {
                 const double2* Ar = Srow + (size_t)q * P;
-                for (int j = sub; j < P; j += 8) {
+#pragma unroll 4
+                for (int j = sub; j < P; j += 16) {
                     const double2 a = Ar[j], vv = p[j];
                     sx = fma(a.x, vv.x, fma(-a.y, vv.y, sx));
                     sy = fma(a.x, vv.y, fma(a.y, vv.x, sy));
                 }
             }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {
+            for (int o = 8; o > 0; o >>= 1) {
                 sx += __shfl_xor_sync(kFull, sx, o);
                 sy += __shfl_xor_sync(kFull, sy, o);
             }
-            if (ok && sub == 0) {
-                Ap[q] = make_double2(sx, sy);
-                const double2 pr = p[r0 + q];
-                pap.x += pr.x * sx + pr.y * sy;
-                pap.y += pr.x * sy - pr.y * sx;
-            }
+            if (q < nr && sub == 0) Ap[q] = make_double2(sx, sy);
         }
-        return pap;
+        __syncthreads();
+    };
+    // r to CTA w and ||r||^2 of this CTA's rows into its slot there
+    auto send_r = [&]() {
+        double rl = 0;
+#pragma unroll
+        for (int c = 0; c < NR; c++) {
+            const int i = lane + 32 * c;
+            if (i >= nr) continue;
+            rf_w[r0 + i] = rr[c];
+            rl += rr[c].x * rr[c].x + rr[c].y * rr[c].y;
+        }
+        rl = warp_sum(rl);
+        if (lane == 0) pb_w[rank] = make_double2(rl, 0);
     };
 
-    (void)matvec();
-    __syncthreads();
-    double rl0 = 0;
-    for (int i = tid; i < nr; i += nt) {
-        const double2 ri = make_double2(b[r0 + i].x - Ap[i].x, b[r0 + i].y - Ap[i].y);
-        for (int c = 0; c < kClusterCta; c++) cl.map_shared_rank(rf, c)[r0 + i] = ri;
-        rl0 += ri.x * ri.x + ri.y * ri.y;
+    matvec();
+    if (w < kClusterCta) {
+#pragma unroll
+        for (int c = 0; c < NR; c++) {
+            const int i = lane + 32 * c;
+            if (i >= nr) continue;
+            xr[c] = p[r0 + i];
+            rr[c] = make_double2(b[r0 + i].x - Ap[i].x, b[r0 + i].y - Ap[i].y);
+        }
+        send_r();
     }
-    push(partB, cta_sum(make_double2(rl0, 0)));
     cl.sync();  // all of r is in every CTA; every CTA has finished reading p = x0
     for (int i = tid; i < P; i += nt) p[i] = rf[i];  // p = r
     __syncthreads();
@@ -749,25 +752,38 @@ __global__ void __cluster_dims__(kClusterCta, 1, 1) __launch_bounds__(256)
     double rs = rsold;
     int itn = 0;
     for (itn = 0; itn < max_it; itn++) {
-        push(partA, cta_sum(matvec()));
-        cl.sync();
-        const double2 pap = total(partA);
-        const double den = pap.x * pap.x + pap.y * pap.y;
-        const double ax = rsold * pap.x / den, ay = -rsold * pap.y / den;
-        double rl = 0;
-        for (int i = tid; i < nr; i += nt) {
-            const double2 pi = p[r0 + i], api = Ap[i];
-            double2 xi = x[i];
-            xi.x += ax * pi.x - ay * pi.y;
-            xi.y += ax * pi.y + ay * pi.x;
-            x[i] = xi;
-            double2 ri = rf[r0 + i];
-            ri.x -= ax * api.x - ay * api.y;
-            ri.y -= ax * api.y + ay * api.x;
-            for (int c = 0; c < kClusterCta; c++) cl.map_shared_rank(rf, c)[r0 + i] = ri;
-            rl += ri.x * ri.x + ri.y * ri.y;
+        matvec();
+        if (w < kClusterCta) {
+            double2 pap = make_double2(0, 0);
+#pragma unroll
+            for (int c = 0; c < NR; c++) {
+                const int i = lane + 32 * c;
+                if (i >= nr) continue;
+                const double2 pr = p[r0 + i], ap = Ap[i];
+                pap.x += pr.x * ap.x + pr.y * ap.y;
+                pap.y += pr.x * ap.y - pr.y * ap.x;
+            }
+            pap.x = warp_sum(pap.x);
+            pap.y = warp_sum(pap.y);
+            if (lane == 0) pa_w[rank] = pap;
         }
-        push(partB, cta_sum(make_double2(rl, 0)));
+        cl.sync();
+        if (w < kClusterCta) {
+            const double2 pap = total(partA);
+            const double den = pap.x * pap.x + pap.y * pap.y;
+            const double ax = rsold * pap.x / den, ay = -rsold * pap.y / den;
+#pragma unroll
+            for (int c = 0; c < NR; c++) {
+                const int i = lane + 32 * c;
+                if (i >= nr) continue;
+                const double2 pi = p[r0 + i], api = Ap[i];
+                xr[c].x += ax * pi.x - ay * pi.y;
+                xr[c].y += ax * pi.y + ay * pi.x;
+                rr[c].x -= ax * api.x - ay * api.y;
+                rr[c].y -= ax * api.y + ay * api.x;
+            }
+            send_r();
+        }
         cl.sync();  // the new r is complete in every CTA
         rs = total(partB).x;
         if (rs < rtol) break;
@@ -779,7 +795,10 @@ __global__ void __cluster_dims__(kClusterCta, 1, 1) __launch_bounds__(256)
         rsold = rs;
         __syncthreads();
     }
-    for (int i = tid; i < nr; i += nt) xg[r0 + i] = x[i];
+    if (w == 0)
+#pragma unroll
+        for (int c = 0; c < NR; c++)
+            if (lane + 32 * c < nr) xg[r0 + lane + 32 * c] = xr[c];
     if (rank == 0 && tid == 0) {
         res->iterations = itn;
         res->residual = rs;
@@ -1059,17 +1078,32 @@ __global__ void unpack_weights(const double2* params, int n, int n_vb, int nh, d
     }
 }
 
+__global__ void widen_kernel(const float2* in, size_t n, double2* out) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float2 v = in[i];
+        out[i] = make_double2(v.x, v.y);
+    }
+}
+
 // ---------------------------------------------------------------- launch --
+cudaError_t launch_widen(const float2* in, size_t n, double2* out, cudaStream_t st) {
+    widen_kernel<<<(unsigned)std::min<size_t>(148 * 8, (n + 255) / 256), 256, 0, st>>>(in, n, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_moments(const void* O, int fp64, const double2* E, int N, int P, int nblk, double2* pd,
                            double2* pf, double2* pe, double2* d, double2* F, double2* emean, cudaStream_t st,
                            const double* w, const double* wsum) {
-    // one column per thread (a single pass over the block's rows) up to 1024
-    // parameters
-    const int thr = std::min(1024, std::max(32, (P + 31) / 32 * 32));
+    // one column per thread: a single pass over the block's rows up to 1024
+    // parameters; above, chunks of 256 columns in their own blocks (19502
+    // parameters of 1000 samples, 15 slices: 0.43 ms of moments and statistics
+    // with each block walking all columns, 0.09 ms here)
+    const int thr = P > 1024 ? 256 : std::max(32, (P + 31) / 32 * 32);
+    const dim3 grid(nblk, (P + thr - 1) / thr);
     if (fp64)
-        moments_partial<double2><<<nblk, thr, 0, st>>>((const double2*)O, E, N, P, pd, pf, pe, w);
+        moments_partial<double2><<<grid, thr, 0, st>>>((const double2*)O, E, N, P, pd, pf, pe, w);
     else
-        moments_partial<float2><<<nblk, thr, 0, st>>>((const float2*)O, E, N, P, pd, pf, pe, w);
+        moments_partial<float2><<<grid, thr, 0, st>>>((const float2*)O, E, N, P, pd, pf, pe, w);
     moments_final<<<(P + 7) / 8, 256, 0, st>>>(pd, pf, pe, nblk, N, P, d, F, emean, wsum);
     return cudaGetLastError();
 }
@@ -1146,7 +1180,7 @@ cudaError_t launch_cg(const double2* A, const double2* b, double2* x, int P, int
     if (csm <= 200 * 1024) {
         cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(cg_cluster), (int)csm);
         if (e != cudaSuccess) return e;
-        cg_cluster<<<kClusterCta, 256, csm, st>>>(A, b, x, P, max_it, rtol, res);
+        cg_cluster<<<kClusterCta, kClusterThreads, csm, st>>>(A, b, x, P, max_it, rtol, res);
         return cudaGetLastError();
     }
     const size_t packed = (packed_size(P) + 4 * (size_t)P) * sizeof(double2);

@@ -277,6 +277,8 @@ cudaError_t launch_cg_mfree(const void* O, int fp64, const double2* d, double no
                             const double2* F, double2* x, const double* diag, const double* max_diag,
                             const ScheduleDev* sch, double r1, double r2, double rd, int max_it, double rtol,
                             const MfreePlan& pl, const MfreeWork& w, CgResultDev* res, cudaStream_t st);
+// FP32 complex values as FP64
+cudaError_t launch_widen(const float2* in, size_t n, double2* out, cudaStream_t st);
 cudaError_t launch_unpack(const double2* params, int n, int n_vb, int nh, double2* vb, double2* hb, double2* W64,
                           float2* W32, float* P32, cudaStream_t st);
 

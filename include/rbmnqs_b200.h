@@ -112,12 +112,14 @@ typedef struct {
     int32_t max_iterations;    /* optimizer.sr.max_iterations (0 = 2P) */
     double rtol;               /* optimizer.sr.rtol (0 = 1e-16) */
     int32_t precision;         /* 0: FP32 psi-ratio math with FP64 theta
-                                     recompute, FP16x3 split-precision tensor-core Gram;
+                                     recompute, FP16x3 split-precision tensor-core
+                                     Gram (FP64 where that is shorter);
                                   1: FP64 throughout */
     int32_t n_updates;         /* rbm n_updates_ (decay_t offset on resume) */
     int32_t gram;              /* S build: 0 = by precision (FP16x3 tensor
-                                  cores when precision is 0, FP64 when 1);
-                                  1 = FP64 CUDA cores in either precision */
+                                  cores when precision is 0, in FP64 where the
+                                  problem is small enough for that to be shorter;
+                                  FP64 when 1); 1 = FP64 in either precision */
     /* Learned proposals (no reference counterpart): 0 = plain Metropolis;
      * 1 = learned_steps moves per sample after every `step` sweeps (step 0:
      * no sweeps, the chains move by learned moves alone).  A move flips one

@@ -1253,7 +1253,7 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
             ck(cudaMemsetAsync(h->dzero.p, 0, h->P * sizeof(double2), h->st), "memset");
             ck(rbmnqs::launch_full_states(h->samples.p, h->n, cfg->full_parallel_bits, h->st), "full states");
         }
-        h->gram_tc = !h->fp64 && cfg->gram == 0 && !h->mfree;
+        h->gram_tc = !h->fp64 && cfg->gram == 0 && !h->mfree && !rbmnqs::gram_fp64_shorter(h->N, h->P);
         require(cfg->solver >= 0 && cfg->solver <= 2, "solver must be 0 (cg), 1 (minresqlp) or 2 (direct)");
         require(cfg->solver != 2 || !h->mfree || h->N <= rbmnqs::kWoodburyMaxN,
                 "the direct solver above " + std::to_string(kDenseMax) + " parameters solves in sample space: at most " +
@@ -2260,6 +2260,11 @@ int rbmnqs_autotune_sr(rbmnqs_handle* h, int32_t* gram_splits, int32_t* cg_kerne
             ck(rbmnqs::gram_tc_set_splits(&h->gtc, bs), "gram splits");
             splits = bs;
             total += best;
+        } else if (!h->mfree) {
+            total += timed([&] {
+                ck(rbmnqs::launch_gram_fp64(h->O.p, h->fp64, dS, h->N, h->P, h->gram_ks, h->part.p, h->Sm.p, h->st),
+                   "gram");
+            });
         }
         // CG kernel on the formed S: the cluster CG against the cooperative
         // one-barrier CG (x restored after each trial)

@@ -1150,6 +1150,15 @@ cudaError_t launch_energy_stats(const double2* E, int N, int n_bins, const doubl
     return cudaGetLastError();
 }
 
+// Three launches (this, its finalize, regularize) against five with the row
+// maxima and the FP16 planes of the tensor-core Gram: what is small is bound by the
+// launches and their latency, and there the FP64 Gram is both exact and shorter.
+// Gram + regularize, us, tensor cores / FP64: N P^2 = 9e4 (256 x 19) 28.8 / 16.4,
+// 4.5e6 (256 x 133) 30.8 / 18.5, 1.8e7 (1024 x 133) 34.8 / 24.6, 2.4e7 (1024 x 153)
+// 35.0 / 26.7; 3.7e7 (8192 x 67) 41.2 / 43.1, 7.2e7 (1024 x 265) 34.8 / 36.9, 1.4e8
+// (8192 x 133) 45.2 / 70.3.
+bool gram_fp64_shorter(int N, int P) { return (double)N * P * P <= 2e7; }
+
 int gram_splits(int N, int P) {
     const int nt = (P + GT - 1) / GT;
     const int tiles = nt * (nt + 1) / 2;

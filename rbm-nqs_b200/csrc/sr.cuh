@@ -49,6 +49,8 @@ cudaError_t launch_energy_stats(const double2* E, int N, int n_bins, const doubl
                                 cudaStream_t st);
 cudaError_t launch_mean(const double2* E, int N, double2* mu, cudaStream_t st);
 int gram_splits(int N, int P);
+// the FP64 Gram takes less time than the tensor-core one (small problems)
+bool gram_fp64_shorter(int N, int P);
 cudaError_t launch_gram_fp64(const void* O, int fp64, const double2* d, int N, int P, int nks, double2* part,
                              double2* S, cudaStream_t st);
 // direct != 0: the direct solver's regularisation (direct_solver.cpp:42-49),

@@ -85,6 +85,30 @@ __device__ __forceinline__ double2 pf_elem(const PfDev& p, uint32_t bits, int i,
     return b < 0 ? make_double2(-v.x, -v.y) : v;
 }
 
+// Change of X(i, f) when site f flips (and site i with it iff ti).  bs is
+// antisymmetric: its row f is read, whose entries for the lanes i lie side by
+// side, in place of column f with a cache line for every two of them.
+__device__ __forceinline__ double2 pf_elem_change(const PfDev& p, uint32_t bits, int i, int f, uint32_t ti) {
+    const int b = -p.bs[f * p.n + i];
+    const int bi = (bits >> i) & 1, bf = (bits >> f) & 1, ci = bi ^ (int)ti, cf = bf ^ 1;
+    const double2* q = p.fs + ((b < 0 ? -b : b) - 1);
+    const double2 a1 = __ldg(&q[(f < i ? (ci << 1) + cf : (cf << 1) + ci) * p.n_indep]);
+    const double2 a0 = __ldg(&q[(f < i ? (bi << 1) + bf : (bf << 1) + bi) * p.n_indep]);
+    const double2 v = zsub(a1, a0);
+    return b < 0 ? make_double2(-v.x, -v.y) : v;
+}
+
+// Butterfly warp sum of a complex value (every lane gets the same result:
+// IEEE addition is commutative).
+__device__ __forceinline__ double2 zwarp_sum(double2 v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    }
+    return v;
+}
+
 // Warp argmax of v (ties: lowest lane).
 __device__ __forceinline__ int warp_argmax(double v) {
     int who = threadIdx.x & 31;
@@ -288,15 +312,12 @@ __device__ __forceinline__ double2 pf_ratio(const PfDev& p, uint32_t bits, const
 #pragma unroll
     for (int q = 0; q < nf; q++) fm |= 1u << fl[q];
     // B: dense columns k < nf (the unit columns nf + k are implicit)
+    double2 b[nf];
 #pragma unroll
     for (int k = 0; k < nf; k++) {
-        double2 b = make_double2(0.0, 0.0);
-        if (lane < n && lane != fl[k]) {
-            const double2 a1 = pf_elem(p, bits, lane, fl[k], (fm >> lane) & 1u, 1);
-            const double2 a0 = pf_elem(p, bits, lane, fl[k], 0, 0);
-            b = zsub(a1, a0);
-        }
-        st.B[lane][k] = b;
+        b[k] = make_double2(0.0, 0.0);
+        if (lane < n && lane != fl[k]) b[k] = pf_elem_change(p, bits, lane, fl[k], (fm >> lane) & 1u);
+        st.B[lane][k] = b[k];
     }
     __syncwarp();
     // this lane's row of X^{-1} B
@@ -314,29 +335,32 @@ __device__ __forceinline__ double2 pf_ratio(const PfDev& p, uint32_t bits, const
 #pragma unroll
     for (int q = 0; q < 2 * nf; q++) st.IB[lane][q] = ib[q];
     __syncwarp();
-    // C^{-1}[r][q], r < q: one pair per lane
+    // C^{-1}[r][q], r < q: one pair per lane.  X^{-1} is antisymmetric to the bit,
+    // so tmp - tmp^T = B^T X^{-1} B: among the dense columns a warp sum per pair,
+    // against a unit column an entry of X^{-1} B.
     const int m2 = 2 * nf;
     const int npairs = m2 * (m2 - 1) / 2;
+    int r = 0, q = lane;
+    while (q >= m2 - 1 - r && r < m2) {
+        q -= m2 - 1 - r;
+        r++;
+    }
+    q += r + 1;
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < nf; k++)
+#pragma unroll
+        for (int l = k + 1; l < nf; l++) {
+            const double2 s = zwarp_sum(zmul(b[k], ib[l]));
+            if (r == k && q == l) acc = s;
+        }
     if (lane < npairs) {
-        int r = 0, q = lane;
-        while (q >= m2 - 1 - r) {
-            q -= m2 - 1 - r;
-            r++;
+        if (r >= nf) {
+            acc = st.IB[fl[r - nf]][q];
+        } else if (q >= nf) {
+            const double2 v = st.IB[fl[q - nf]][r];
+            acc = make_double2(-v.x, -v.y);
         }
-        q += r + 1;
-        // (tmp - tmp^T)[r][q] = 1/2 sum_t (B[t][r] IB[t][q] - B[t][q] IB[t][r])
-        double2 acc = make_double2(0.0, 0.0);
-        if (r < nf) {
-            for (int t = 0; t < n; t++) acc = zfma(st.B[t][r], st.IB[t][q], acc);
-        } else {
-            acc = zadd(acc, st.IB[fl[r - nf]][q]);
-        }
-        if (q < nf) {
-            for (int t = 0; t < n; t++) acc = zsub(acc, zmul(st.B[t][q], st.IB[t][r]));
-        } else {
-            acc = zsub(acc, st.IB[fl[q - nf]][r]);
-        }
-        acc = zscale(acc, 0.5);
         // C0: C(nf + k, k) = 1 and C(k, l) = a(f_k, f_l) - a'(f_k, f_l), l < k
         if (r < nf && q == nf + r) acc.x -= 1.0;
         if (q < nf) {
@@ -541,17 +565,6 @@ __device__ __forceinline__ void pf_fresh_circ(const PfDev& p, uint32_t bits, int
     __syncwarp();
 }
 
-// Butterfly warp sum of a complex value (every lane gets the same result:
-// IEEE addition is commutative).
-__device__ __forceinline__ double2 zwarp_sum(double2 v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
-    }
-    return v;
-}
-
 // Pairs of the 2 NF x 2 NF matrix C^{-1} (r < q), every lane: NF = 1: c[0]
 // = (0, 1); NF = 2: c = (0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3).
 template <int NF> struct PfPairs {
@@ -560,10 +573,19 @@ template <int NF> struct PfPairs {
 
 // psi ratio factor of the Pfaffian for flipping sites fl[0..NF) with X^{-1}
 // in circulant form (the same rank-2m formula as pf_ratio).  Lane t holds
-// row t of B and of X^{-1} B (ib), so each entry of C^{-1} is one warp sum
-// of lane products plus entries of X^{-1} B on the flipped sites' lanes.
+// row t of B and of X^{-1} B (ib).  X^{-1} is antisymmetric, so C^{-1} - C0 =
+// B^T X^{-1} B: one warp sum of lane products for the two dense columns, and
+// entries of X^{-1} B on the flipped sites' lanes against the unit columns
+// (tmp - tmp^T, which holds each entry twice, takes five warp sums).
 // Leaves X^{-1} B in st.IB (and this lane's row in ib) and C^{-1} in cp for
 // pf_accept_circ.  Warp-collective.
+//
+// What bounds the sweep: shared-memory wavefronts (53 % of peak before, FP64 21 %)
+// and instruction fetch (2.3 of 8.9 stalled warps per issue), since the warps of an
+// SM stand at different places of a long loop.  So the loops over d are unrolled
+// only as far as two loads are in flight.  2048 chains of 32 spins, 64 sweeps, ms:
+// five warp sums and column reads of bs, unroll 4 11.8; one warp sum and row reads
+// 9.95; unroll 2 9.2 (unroll 1 9.6).
 template <int NF>
 __device__ __forceinline__ double2 pf_ratio_circ(const PfDev& p, uint32_t bits, const int* fl, int lane,
                                                  PfSweepStage& st, const double2* Cx, double2 (&ib)[2 * NF],
@@ -577,11 +599,7 @@ __device__ __forceinline__ double2 pf_ratio_circ(const PfDev& p, uint32_t bits, 
 #pragma unroll
     for (int k = 0; k < NF; k++) {
         b[k] = make_double2(0.0, 0.0);
-        if (lane < n && lane != fl[k]) {
-            const double2 a1 = pf_elem(p, bits, lane, fl[k], (fm >> lane) & 1u, 1);
-            const double2 a0 = pf_elem(p, bits, lane, fl[k], 0, 0);
-            b[k] = zsub(a1, a0);
-        }
+        if (lane < n && lane != fl[k]) b[k] = pf_elem_change(p, bits, lane, fl[k], (fm >> lane) & 1u);
         st.BT[k][lane] = b[k];
     }
     __syncwarp();
@@ -589,14 +607,14 @@ __device__ __forceinline__ double2 pf_ratio_circ(const PfDev& p, uint32_t bits, 
     double2 up[NF], dn[NF];
 #pragma unroll
     for (int k = 0; k < NF; k++) up[k] = dn[k] = make_double2(0.0, 0.0);
-#pragma unroll 4
+#pragma unroll 2
     for (int d = 1; d <= 16; d++) {
         const int j = (lane + d) & 31;
         const double2 x = Cx[(d - 1) * kPfMaxSites + lane];
 #pragma unroll
         for (int k = 0; k < NF; k++) up[k] = zfma(x, st.BT[k][j], up[k]);
     }
-#pragma unroll 5
+#pragma unroll 3
     for (int d = 1; d <= 15; d++) {
         const int j = (lane - d) & 31;
         const double2 x = Cx[(d - 1) * kPfMaxSites + j];
@@ -613,30 +631,22 @@ __device__ __forceinline__ double2 pf_ratio_circ(const PfDev& p, uint32_t bits, 
     // X^{-1} B entries on the flipped sites' lanes
     auto at = [&](int q, int site) { return zshfl(ib[q], site); };
     if constexpr (NF == 1) {
-        // (0, 1): (sum_t B_t0 IB_t1 - IB_{f0,0}) / 2 - 1
-        const double2 s = zwarp_sum(zmul(b[0], ib[1]));
-        double2 c = zscale(zsub(s, at(0, fl[0])), 0.5);
-        c.x -= 1.0;
-        cp.c[0] = c;
-        return make_double2(-c.x, -c.y);  // (-1)^{m(m+1)/2}, m = 1
+        // (0, 1): -IB_{f0,0} - 1
+        const double2 i00 = at(0, fl[0]);
+        cp.c[0] = make_double2(-i00.x - 1.0, -i00.y);
+        return make_double2(i00.x + 1.0, i00.y);  // (-1)^{m(m+1)/2}, m = 1
     } else {
-        const double2 s01 = zwarp_sum(zsub(zmul(b[0], ib[1]), zmul(b[1], ib[0])));
-        const double2 s02 = zwarp_sum(zmul(b[0], ib[2]));
-        const double2 s03 = zwarp_sum(zmul(b[0], ib[3]));
-        const double2 s12 = zwarp_sum(zmul(b[1], ib[2]));
-        const double2 s13 = zwarp_sum(zmul(b[1], ib[3]));
+        const double2 s01 = zwarp_sum(zmul(b[0], ib[1]));
         const double2 i00 = at(0, fl[0]), i01 = at(1, fl[0]), i03 = at(3, fl[0]);
-        const double2 i10 = at(0, fl[1]), i11 = at(1, fl[1]), i12 = at(2, fl[1]);
+        const double2 i10 = at(0, fl[1]), i11 = at(1, fl[1]);
         // C0: C(k, l) = a(f_k, f_l) - a'(f_k, f_l) below the diagonal block
         const double2 d01 = zsub(pf_elem(p, bits, fl[1], fl[0], 0, 0), pf_elem(p, bits, fl[1], fl[0], 1, 1));
-        cp.c[0] = zsub(zscale(s01, 0.5), d01);
-        cp.c[1] = zscale(zsub(s02, i00), 0.5);
-        cp.c[1].x -= 1.0;
-        cp.c[2] = zscale(zsub(s03, i10), 0.5);
-        cp.c[3] = zscale(zsub(s12, i01), 0.5);
-        cp.c[4] = zscale(zsub(s13, i11), 0.5);
-        cp.c[4].x -= 1.0;
-        cp.c[5] = zscale(zsub(i03, i12), 0.5);
+        cp.c[0] = zsub(s01, d01);
+        cp.c[1] = make_double2(-i00.x - 1.0, -i00.y);
+        cp.c[2] = make_double2(-i10.x, -i10.y);
+        cp.c[3] = make_double2(-i01.x, -i01.y);
+        cp.c[4] = make_double2(-i11.x - 1.0, -i11.y);
+        cp.c[5] = i03;
         const double2 pf = zadd(zsub(zmul(cp.c[0], cp.c[5]), zmul(cp.c[1], cp.c[4])), zmul(cp.c[2], cp.c[3]));
         return make_double2(-pf.x, -pf.y);  // (-1)^{m(m+1)/2}, m = 2
     }
@@ -671,7 +681,7 @@ __device__ __forceinline__ void pf_accept_circ(int lane, const PfSweepStage& st,
     }
     __syncwarp();  // st.IB of every lane
     if (lane < n) {
-#pragma unroll 4
+#pragma unroll 2
         for (int d = 1; d <= 16; d++) {
             const int j = (lane + d) & 31;
             double2 acc = Cx[(d - 1) * kPfMaxSites + lane];

@@ -629,7 +629,6 @@ def run_forms(args, rank, world, local):
         taus2.append(st["tau"])
     torch.cuda.synchronize()
     t2_ms = sum(a.elapsed_time(b) for a, b in ev2)
-    mufu = rbmnqs.probe_mufu() if rank == 0 else 0.0
     T = learned.n_hidden * learned.n_symm
     P = learned.n_params
     del learned
@@ -655,11 +654,12 @@ def run_forms(args, rank, world, local):
     value = world * args.steps * N / (1.0 + 2.0 * L["tau"]) / (t_learned_ms * 1e-3)
     e2e = world * args.steps * N / (1.0 + 2.0 * float(np.mean(taus2))) / (t2_ms * 1e-3)
     # roofline of the dominant kernel (the E_loc / O_k evaluation): every
-    # off-diagonal term (the x and y bonds, n / 2 each) evaluates ln cosh of
-    # all T theta entries of theta', each one ex2, one sin and one cos (the
-    # per-four lg2 and rsqrt not counted)
+    # off-diagonal term (the x and y bonds, n / 2 each) takes a complex addition
+    # and a complex multiplication per theta entry: six operations of the FMA
+    # pipe (128 lanes per SM, 148 SMs)
     terms = n
-    ops = float(N) * terms * T * 3.0
+    ops = float(N) * terms * T * 6.0
+    fma = 148 * 128 * 1e6 * ((clocks or {}).get("sm_max_mhz") or 1965)
     eval_ms = L["stage_ms_per_epoch"]["eval"]
     achieved = ops / (eval_ms * 1e-3)
     sweep_ms = L["stage_ms_per_epoch"]["sampler"]
@@ -690,12 +690,13 @@ def run_forms(args, rank, world, local):
         "delta_energy_per_site_learned_vs_plain_fp64": {
             "value": L["energy_per_site"] - out["plain_fp64"]["energy_per_site"],
             "stderr": float(np.hypot(L["energy_per_site_stderr"], out["plain_fp64"]["energy_per_site_stderr"]))},
-        "roofline": {"bound": "mufu", "kernel": "eloc_kernel", "achieved": achieved / 1e9, "peak": mufu / 1e9,
-                     "unit": "Gop/s (MUFU)", "frac": achieved / mufu,
-                     "peak_source": "measured in this run by rbmnqs_probe_mufu (no MUFU figure in "
-                                    "MEASURED_PEAKS.json)",
+        "roofline": {"bound": "fp32", "kernel": "eloc_sym_kernel", "achieved": achieved / 1e9, "peak": fma / 1e9,
+                     "unit": "Gop/s (FP32 FMA pipe)", "frac": achieved / fma,
+                     "peak_source": "148 SMs x 128 lanes at the maximum SM clock (no FP32 figure in "
+                                    "MEASURED_PEAKS.json); the kernel's own bound is shared-memory wavefronts",
                      "algorithmic_ops_per_launch": ops,
-                     "ops_per_unit": "3 MUFU (ex2, sin, cos) per theta entry per off-diagonal term per sample: "
+                     "ops_per_unit": "6 FP32 operations (z + q and the running product) per theta entry per "
+                                     "off-diagonal term per sample: "
                                      f"{N} samples x {terms} terms x {T} entries",
                      "traffic": ELOC_DRAM_BYTES.get(args.workload),
                      "traffic_source": ELOC_TRAFFIC_SOURCE,

@@ -318,7 +318,7 @@ struct rbmnqs_handle {
 
     DevBuf<double2> params, vb, hb, W64, x;
     DevBuf<float2> W32;
-    DevBuf<float> P32;  // exp(+-4 W) for the screened FP32 sweep
+    DevBuf<float> P32;  // exp(+-4 W) for the screened sweep
     DevBuf<uint8_t> perm, inv, orbit;
     DevBuf<uint8_t> wrank;  // row order of W in the FP32 evaluation kernel (symmetric machines)
     DevBuf<rbmnqs::OpDev> ops;

@@ -301,7 +301,7 @@ __device__ __forceinline__ double2 pf_small(PfStage& st, int m2, int lane) {
 // configuration `bits` (pfaffian::psi_over_psi via update_context).  Xi(t)
 // returns X^{-1}[lane][t] (t a compile-time index when unrolled), Xcol(f)
 // returns X^{-1}[lane][f] for a runtime f.  Leaves X^{-1}B in st.IB and in
-// ib (this lane's row) and C^{-1} in st.C for pf_accept.  Warp-collective.
+// ib (this lane's row) and C^{-1} in st.C.  Warp-collective.
 template <int NF, typename XI, typename XCOL>
 __device__ __forceinline__ double2 pf_ratio(const PfDev& p, uint32_t bits, const int* fl, int lane, PfStage& st,
                                             XI Xi, XCOL Xcol, double2 (&ib)[2 * kPfMaxFlips]) {
@@ -373,52 +373,6 @@ __device__ __forceinline__ double2 pf_ratio(const PfDev& p, uint32_t bits, const
     const double2 pf = pf_small(st, m2, lane);
     const int sgn = ((nf * (nf + 1) / 2) & 1) ? -1 : 1;
     return sgn > 0 ? pf : make_double2(-pf.x, -pf.y);
-}
-
-// X^{-1} update after an accepted move of nf <= 2 flips (pfaffian.cpp:360-386):
-// with Ca = (C^{-1})^{-1} (antisymmetric), X^{-1} += (X^{-1}B) Ca (X^{-1}B)^T,
-// which equals the reference's T2 - T2^T with T2 = X^{-1}B Ca (X^{-1}B)^T / 2.
-// Uses st.C / st.IB / ib from the pf_ratio call of the same proposal; lane i
-// updates row i of A.
-__device__ __forceinline__ void pf_accept(int nf, int lane, const PfStage& st, const double2 (&ib)[2 * kPfMaxFlips],
-                                          double2* A, int n) {
-    double2 Ca[4][4];
-    const auto& C = st.C;
-    if (nf == 1) {
-        const double2 ic = zrcp(C[0][1]);
-        Ca[0][0] = Ca[1][1] = make_double2(0.0, 0.0);
-        Ca[0][1] = make_double2(-ic.x, -ic.y);
-        Ca[1][0] = ic;
-    } else {
-        const double2 c01 = C[0][1], c02 = C[0][2], c03 = C[0][3], c12 = C[1][2], c13 = C[1][3], c23 = C[2][3];
-        const double2 ip = zrcp(zadd(zsub(zmul(c01, c23), zmul(c02, c13)), zmul(c03, c12)));
-        auto s = [&](double2 v, double sg) { const double2 w = zmul(v, ip); return make_double2(sg * w.x, sg * w.y); };
-        Ca[0][0] = Ca[1][1] = Ca[2][2] = Ca[3][3] = make_double2(0.0, 0.0);
-        Ca[0][1] = s(c23, -1.0); Ca[0][2] = s(c13, 1.0); Ca[0][3] = s(c12, -1.0);
-        Ca[1][0] = s(c23, 1.0); Ca[1][2] = s(c03, -1.0); Ca[1][3] = s(c02, 1.0);
-        Ca[2][0] = s(c13, -1.0); Ca[2][1] = s(c03, 1.0); Ca[2][3] = s(c01, -1.0);
-        Ca[3][0] = s(c12, 1.0); Ca[3][1] = s(c02, -1.0); Ca[3][2] = s(c01, 1.0);
-    }
-    const int m2 = 2 * nf;
-    double2 t1[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int t = 0; t < 4; t++)
-            if (t < m2 && q < m2) acc = zfma(ib[t], Ca[t][q], acc);
-        t1[q] = acc;
-    }
-    if (lane < n) {
-        for (int j = 0; j < n; j++) {
-            double2 acc = A[lane * kPfLd + j];
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (q < m2) acc = zfma(t1[q], st.IB[j][q], acc);
-            A[lane * kPfLd + j] = acc;
-        }
-    }
-    __syncwarp();
 }
 
 // log Pf(X) of configuration `bits` (pfaffian.cpp:294-296, PFAPACK skpf10
@@ -652,7 +606,8 @@ __device__ __forceinline__ double2 pf_ratio_circ(const PfDev& p, uint32_t bits, 
     }
 }
 
-// X^{-1} update after an accepted move (pf_accept in circulant form): with
+// X^{-1} update after an accepted move (pfaffian.cpp:360-386): X^{-1} +=
+// (X^{-1}B) Ca (X^{-1}B)^T, the reference's T2 - T2^T.  With
 // Ca = (C^{-1})^{-1}, t1 = (row i of X^{-1} B) Ca and
 // X^{-1}(i, i + d) += t1 . (row i + d of X^{-1} B), d = 1..16.
 template <int NF>

@@ -11,8 +11,10 @@
 // lanes with warp shuffles; every lane holds the same configuration bits and
 // takes the same accept/reject branch.  theta is recomputed in FP64 from the
 // configuration after every sweep (mixed-precision scheme), so FP32
-// drift never outlives one sweep.  With the Pfaffian factor (sites <= 32) each
-// lane also holds its row of X^{-1} in FP64 registers (pfaffian.cuh).
+// drift never outlives one sweep.  With the Pfaffian factor (sites <= 32) the
+// warp also holds X^{-1} in shared memory (pfaffian.cuh).  FP64 sweeps, and FP32
+// sweeps of 16 entries per lane, screen the proposals by products
+// (sampler_screen.cuh).
 #include <algorithm>
 #include <map>
 #include <mutex>

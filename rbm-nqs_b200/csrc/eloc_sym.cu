@@ -20,12 +20,20 @@
 //
 // The products carry their exponents as integers: a lane's product over its
 // entries is scaled to a leading one, mantissas multiply and exponents add in
-// the warp's butterfly, and exp() joins them in FP64, 32 terms at a time.  A
-// lane whose product leaves the FP32 range (an entry of vanishing amplitude,
-// activations far beyond trained ones, |4 W| > 60 in a row, non-finite
-// weights) sends its configuration to ratio_slow(), the ln cosh sums in FP64.
+// the warp's butterfly, and exp() joins them in FP64, 32 terms at a time.
 // Configurations with Re sum theta < 0 take -theta (cosh is even), which keeps
 // |z| below one on average.
+//
+// Range.  z and q are each rounded once from FP64, over their whole range (z is
+// exp(-2 theta) itself, not 1 - (1 - z): a flip that cancels a saturated theta
+// leaves z + q as small as z).  A lane multiplies its entries in two chains of E /
+// 2; a chain that ends above 2^-116 F^(E/2 - 1), F a bound on |z + q| over the
+// configuration's entries and the block's table, has not been below 2^-116 on its
+// way, and one that overflowed ends as infinity or NaN.  A configuration with a
+// chain outside that range takes term_product_scaled() from that term on, which
+// scales after every factor.  Factors that FP32 does not hold, or that are zero
+// (|z| > e^68, |4 W| > 60 in a row, q outside 2^+-86, non-finite weights) send
+// the configuration to ratio_slow(), the ln cosh sums in FP64.
 //
 // Layout as in eloc.cuh: groups of KB hidden units with one symmetry index s,
 // lane l owns the groups l + 32 j; entries in pairs, real and imaginary parts
@@ -49,7 +57,7 @@ namespace {
 using namespace eloc;
 
 struct SymLayout {
-    int w64, perm, inv, cls, q, base, terms, diag, vals, vb, site, warp0, warp_bytes, total;
+    int w64, perm, inv, cls, q, base, terms, diag, vals, vb, site, qmax, warp0, warp_bytes, total;
     int ws64;    // row stride of the FP64 W copy (double2)
     int qs, qp;  // row and pattern strides of q (bytes)
 };
@@ -81,6 +89,7 @@ __host__ __device__ inline SymLayout sym_layout(const MachineDev& m, const TermT
     L.vals = take(tt.n_vals * 16);
     L.vb = take(m.n_vb * 16);
     L.site = take((m.n + 1) * 16);
+    L.qmax = take(4);
     L.warp0 = off;
     const int scratch = warps * L.warp_bytes, factors = m.n * m.nh * 32;
     off += a16(scratch > factors ? scratch : factors);
@@ -164,24 +173,14 @@ __device__ __noinline__ double2 ratio_slow(const MachineDev* __restrict__ md, in
     return make_double2(ex, ey);
 }
 
-// Product over the lane's entries of (z + q): zr, zi pairs; qb the pattern's
-// table (byte address), cb the term's row of the tuple table.
-template <int KB, int NG>
-__device__ __forceinline__ float2 term_product(const float2 (&zr)[KB * NG / 2], const float2 (&zi)[KB * NG / 2],
-                                               uint32_t qb, uint32_t cb, const uint32_t (&s2)[NG],
-                                               const uint32_t (&ko)[NG]) {
-    float2 Px, Py;
-    auto mul = [&](int p, float2 qr, float2 qi) {
-        const float2 fr = __fadd2_rn(zr[p], qr), fi = __fadd2_rn(zi[p], qi);
-        if (p == 0) {
-            Px = fr;
-            Py = fi;
-        } else {
-            const float2 nx = __ffma2_rn(Px, fr, __fmul2_rn(make_float2(-Py.x, -Py.y), fi));
-            Py = __ffma2_rn(Px, fi, __fmul2_rn(Py, fr));
-            Px = nx;
-        }
-    };
+// The factors (z + q) of the lane's entries, in pairs, to mul(pair, real parts,
+// imaginary parts): zr, zi pairs; qb the pattern's table (byte address), cb the
+// term's row of the tuple table.
+template <int KB, int NG, typename F>
+__device__ __forceinline__ void term_factors(const float2 (&zr)[KB * NG / 2], const float2 (&zi)[KB * NG / 2],
+                                             uint32_t qb, uint32_t cb, const uint32_t (&s2)[NG],
+                                             const uint32_t (&ko)[NG], F&& factor) {
+    auto mul = [&](int p, float2 qr, float2 qi) { factor(p, __fadd2_rn(zr[p], qr), __fadd2_rn(zi[p], qi)); };
     if constexpr (KB == 4) {
 #pragma unroll
         for (int j = 0; j < NG; j++) {
@@ -204,11 +203,10 @@ __device__ __forceinline__ float2 term_product(const float2 (&zr)[KB * NG / 2], 
             mul(j / 2, make_float2(v0.x, v1.x), make_float2(v0.y, v1.y));
         }
     }
-    return make_float2(Px.x * Px.y - Py.x * Py.y, Px.x * Py.y + Py.x * Px.y);
 }
 
-// Scale p to a leading one: p 2^-e, e its exponent.  False outside 2^-100 ..
-// 2^100 (and for NaN).
+// Scale p to a leading one: p 2^-e, e its exponent.  False outside 2^-116 ..
+// 2^116 (and for NaN).
 __device__ __forceinline__ bool split(float2& p, int& e) {
     const float mx = fmaxf(fabsf(p.x), fabsf(p.y));
     const uint32_t b = __float_as_uint(mx) & 0x7f800000u;
@@ -216,7 +214,52 @@ __device__ __forceinline__ bool split(float2& p, int& e) {
     const float sc = __uint_as_float(0x7f000000u - b);
     p.x *= sc;
     p.y *= sc;
-    return mx >= 7.8886091e-31f && mx <= 1.2676506e30f && p.x == p.x && p.y == p.y;
+    return mx >= 1.2037062e-35f && mx <= 8.3076750e34f && p.x == p.x && p.y == p.y;
+}
+
+// Product over the lane's entries of (z + q), scaled to a leading one.  False
+// where a chain ends below `low` or the product leaves the range of split().
+template <int KB, int NG>
+__device__ __forceinline__ bool term_product(const float2 (&zr)[KB * NG / 2], const float2 (&zi)[KB * NG / 2],
+                                             uint32_t qb, uint32_t cb, const uint32_t (&s2)[NG],
+                                             const uint32_t (&ko)[NG], float low, float2& u, int& e) {
+    float2 Px, Py;
+    term_factors<KB, NG>(zr, zi, qb, cb, s2, ko, [&](int p, float2 fr, float2 fi) {
+        if (p == 0) {
+            Px = fr;
+            Py = fi;
+        } else {
+            const float2 nx = __ffma2_rn(Px, fr, __fmul2_rn(make_float2(-Py.x, -Py.y), fi));
+            Py = __ffma2_rn(Px, fi, __fmul2_rn(Py, fr));
+            Px = nx;
+        }
+    });
+    u = make_float2(Px.x * Px.y - Py.x * Py.y, Px.x * Py.y + Py.x * Px.y);
+    const float lo = fminf(fmaxf(fabsf(Px.x), fabsf(Py.x)), fmaxf(fabsf(Px.y), fabsf(Py.y)));
+    return split(u, e) & (lo >= low);
+}
+
+// The same, scaled after every factor: false only where a factor is zero or
+// outside split()'s range.
+template <int KB, int NG>
+__device__ __forceinline__ bool term_product_scaled(const float2 (&zr)[KB * NG / 2], const float2 (&zi)[KB * NG / 2],
+                                                    uint32_t qb, uint32_t cb, const uint32_t (&s2)[NG],
+                                                    const uint32_t (&ko)[NG], float2& u, int& e) {
+    bool ok = true;
+    u = make_float2(1.f, 0.f);
+    e = 0;
+    term_factors<KB, NG>(zr, zi, qb, cb, s2, ko, [&](int, float2 fr, float2 fi) {
+        float2 f[2] = {make_float2(fr.x, fi.x), make_float2(fr.y, fi.y)};
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            int ef, eu;
+            ok &= split(f[i], ef);
+            u = cmul(u, f[i]);
+            ok &= split(u, eu);
+            e += ef + eu;
+        }
+    });
+    return ok;
 }
 
 // Butterfly reduce-scatter of KT per-lane partials (mantissas multiply,
@@ -278,6 +321,7 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
     double2* sVals = reinterpret_cast<double2*>(smem + L.vals);
     double2* sVb = reinterpret_cast<double2*>(smem + L.vb);
     double2* sSite = reinterpret_cast<double2*>(smem + L.site);  // 2 sum_e W_fe; entry n: sum_e hb_e
+    unsigned* sQmax = reinterpret_cast<unsigned*>(smem + L.qmax);  // largest |q| component, a float's bits
     double2* fac = reinterpret_cast<double2*>(smem + L.warp0);   // exp(-4 W), exp(4 W) per (row, k)
     auto rk = [&](int r) { return a.wrank ? (int)a.wrank[r] : r; };
     for (int i = tid; i < n * nh; i += nthr) {
@@ -306,8 +350,10 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
     for (int i = tid; i < n_diag; i += nthr) sDiag[i] = a.tt.diag[i];
     for (int i = tid; i < a.tt.n_vals; i += nthr) sVals[i] = a.tt.vals[i];
     for (int i = tid; i < n_vb; i += nthr) sVb[i] = m.vb[i];
+    if (tid == 0) *sQmax = 0;
     __syncthreads();
     // q of every tuple, hidden unit and spin pattern (bit set: spin down)
+    float qmax = 0.f;
     for (int i = tid; i < (n_cls + 1) * nh; i += nthr) {
         const int c = i / nh, k = i - c * nh, kk = k % KB, k0 = k - kk;
         const uint8_t* tup = a.tt.tup + 8 * c;
@@ -321,10 +367,13 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
             const double mx = fmax(fabs(v.x), fabs(v.y));
             const bool ok = mx < 7.7e25 && mx > 1.3e-26;
             const float bad = __int_as_float(0x7fc00000);
+            if (ok) qmax = fmaxf(qmax, (float)mx);
             *reinterpret_cast<float*>(row) = ok ? (float)v.x : bad;
             *reinterpret_cast<float*>(row + (KB == 1 ? 4 : 8)) = ok ? (float)v.y : bad;
         }
     }
+    const unsigned qw = __reduce_max_sync(kFull, __float_as_uint(qmax));
+    if ((tid & 31) == 0) atomicMax(sQmax, qw);
     for (int t = tid; t < T; t += nthr) {
         const int k = t % nh, s = t / nh;
         double2 acc = m.hb[k];
@@ -386,7 +435,16 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
         // theta in FP64 into the warp's scratch, z = exp(-+2 theta) to FP32
         // pairs, and the lane's product of 1 + z
         float2 zr[NP], zi[NP];
+        float zmax = 0.f;
         double2 D = make_double2(1, 0);
+        int ec = 0;  // the product's exponent, apart from D
+        auto lead = [&]() {  // D to a leading one
+            const int hi = (__double2hiint(fmax(fabs(D.x), fabs(D.y))) >> 20) & 0x7ff;
+            const double sc = __hiloint2double((min(max(2046 - hi, 1), 2046)) << 20, 0);
+            D.x *= sc;
+            D.y *= sc;
+            ec += hi - 1023;
+        };
         double lre = 0, lim = 0;  // sum ln cosh theta (principal values), ln 2 per entry left out
 #pragma unroll
         for (int j = 0; j < NG; j++) {
@@ -418,28 +476,30 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                 const int e = j * KB + i;
                 double zx = 0, zy = 0;
                 if (ok) {
-                    // the terms of ctanh_r, shared with z
                     const double x = acc[i].x, aa = fabs(x);
-                    const double omz = -expm1(-2.0 * aa), w = 1.0 - omz;
                     double s, c;
                     sincos(acc[i].y, &s, &c);
-                    const double X = (1.0 + w) * c, Y = omz * s;
-                    if constexpr (LP) {
-                        lre += aa + 0.5 * log(X * X + Y * Y);
-                        lim += atan2(copysign(omz, x) * s, X);
+                    if (LP || a.O) {  // the terms of ctanh_r
+                        const double omz = -expm1(-2.0 * aa), w = 1.0 - omz;
+                        const double X = (1.0 + w) * c, Y = omz * s;
+                        if constexpr (LP) {
+                            lre += aa + 0.5 * log(X * X + Y * Y);
+                            lim += atan2(copysign(omz, x) * s, X);
+                        }
+                        if (a.O) {
+                            const double inv = 1.0 / (X * X + Y * Y);
+                            tn[t0 + i] = make_float2((float)(copysign(omz * (1.0 + w), x) * inv),
+                                                     (float)(4.0 * w * s * c * inv));
+                        }
                     }
-                    if (a.O) {
-                        const double inv = 1.0 / (X * X + Y * Y);
-                        tn[t0 + i] = make_float2((float)(copysign(omz * (1.0 + w), x) * inv),
-                                                 (float)(4.0 * w * s * c * inv));
-                    }
-                    // |z| = exp(-2 |x|), or its inverse (capped at e^40, where
-                    // z + q = z to FP32 precision) on the other side
-                    const bool big = (x < 0) != neg && x != 0;
-                    const double r = big ? 1.0 / fmax(w, 4.248354255291589e-18) : w;
+                    // z; beyond e^68, where a factor's product may leave FP32, NaN
+                    const double v = neg ? 2.0 * x : -2.0 * x;
+                    const double r = v <= 68.0 ? exp(v) : __longlong_as_double(0x7ff8000000000000ll);
                     zx = r * (c * c - s * s);
                     zy = (neg ? 2.0 : -2.0) * r * s * c;
+                    zmax = fmaxf(zmax, (float)r);
                     D = cmul(D, make_double2(1.0 + zx, zy));
+                    if (e % 8 == 7) lead();
                 }
                 if (e & 1) {
                     zr[e >> 1].y = (float)zx;
@@ -466,17 +526,11 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
         }
         if (a.eloc) {
             double ex = 0.0, ey = 0.0;
-            // C = prod 1 / (1 + z) = C 2^ec
-            int ec;
+            // prod 1 / (1 + z) = D 2^-ec
+            bool safe;
             {
-                auto lead = [&]() {  // D to a leading one
-                    const int hi = (__double2hiint(fmax(fabs(D.x), fabs(D.y))) >> 20) & 0x7ff;
-                    const double sc = __hiloint2double((min(max(2046 - hi, 1), 2046)) << 20, 0);
-                    D.x *= sc;
-                    D.y *= sc;
-                    return hi - 1023;
-                };
-                ec = lead();
+                lead();
+                safe = __all_sync(kFull, D.x != 0.0 || D.y != 0.0);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     double2 w;
@@ -489,7 +543,12 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                 D.x *= inv;
                 D.y *= -inv;
             }
-            bool safe = true;
+            // the lowest end of a chain that has stayed in range (NaN in z: any)
+            const uint32_t fb = __float_as_uint(2.83f * (__uint_as_float(*sQmax) +
+                                                         __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(zmax)))));
+            const int lexp = (NP - 1) * ((int)(fb >> 23) - 126) - 116;
+            bool scaled = lexp > 8;
+            const float low = __uint_as_float((uint32_t)(max(min(lexp, 8), -116) + 127) << 23);
             for (int c0 = 0; c0 < n_terms && safe; c0 += 32) {
                 // the lane's term: its pattern table and exponent
                 const int tl = min(c0 + lane, n_terms - 1);
@@ -509,7 +568,7 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                 const uint32_t pb = qa + (uint32_t)(pat * L.qp);
                 int Re = 0;
                 float2 U = make_float2(0.f, 0.f);
-                for (int r = 0; r < 32 / KT && c0 + r * KT < n_terms; r++) {
+                for (int r = 0; r < 32 / KT && c0 + r * KT < n_terms && !scaled; r++) {
                     int pe[KT];
                     float2 pu[KT];
                     bool ok = true;
@@ -517,11 +576,10 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                     for (int q = 0; q < KT; q++) {
                         const uint32_t qb = __shfl_sync(kFull, pb, r * KT + q);
                         const int ti = min(c0 + r * KT + q, n_terms - 1);
-                        pu[q] = term_product<KB, NG>(zr, zi, qb, ca + 2u * (uint32_t)(ti * SP), s2, ko);
-                        ok &= split(pu[q], pe[q]);
+                        ok &= term_product<KB, NG>(zr, zi, qb, ca + 2u * (uint32_t)(ti * SP), s2, ko, low, pu[q], pe[q]);
                     }
                     if (!__all_sync(kFull, ok)) {
-                        safe = false;
+                        scaled = true;
                         break;
                     }
                     int R;
@@ -534,6 +592,22 @@ __global__ void __launch_bounds__(32 * eloc_warps(KB* NG), eloc_min_blocks(KB* N
                     if (lane / KT == r) {
                         Re = er;
                         U = make_float2(vx, vy);
+                    }
+                }
+                if (scaled) {  // one term at a time
+#pragma unroll 1
+                    for (int t = c0; t < min(c0 + 32, n_terms) && safe; t++) {
+                        const uint32_t qb = __shfl_sync(kFull, pb, t - c0);
+                        float2 V;
+                        int R;
+                        const bool ok = term_product_scaled<KB, NG>(zr, zi, qb, ca + 2u * (uint32_t)(t * SP), s2, ko, V, R);
+                        safe = __all_sync(kFull, ok);
+                        R = __reduce_add_sync(kFull, R);
+                        V = warp_cprod(V);
+                        if (lane == t - c0) {
+                            Re = R;
+                            U = V;
+                        }
                     }
                 }
                 if (safe && c0 + lane < n_terms) {

@@ -290,7 +290,8 @@ int rbmnqs_timing_reset(rbmnqs_handle* h, int32_t enable);
 /* Launch-shape autotuner: times the sweep kernel over `sweeps` sweeps (one
  * recorded sample) for one and (where the expanded-table path allows it)
  * two chains per warp, each with up to five warps-per-block caps, and the
- * evaluation kernel for 1..8 warps per block;
+ * evaluation kernel for 1..8 warps per block (full enumeration: the
+ * evaluation alone, sampler_ms 0);
  * keeps the fastest of each (the session's chains, weights and statistics
  * are left as they were; the epoch graph is re-captured).  No reference
  * counterpart (the reference has no launch shapes).  Outputs may be NULL. */

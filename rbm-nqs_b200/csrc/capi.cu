@@ -2159,7 +2159,9 @@ int rbmnqs_autotune(rbmnqs_handle* h, int32_t sweeps, int32_t* sampler_wpb, int3
         args.spc = 1;
         args.step = 1;
         args.warmup = sweeps - 1;
-        if (!h->pf_n) {  // the Pfaffian buffers are sized for the planned shape
+        // the Pfaffian buffers are sized for the planned shape; full enumeration
+        // does not sweep (its list of states is where a sweep records)
+        if (!h->pf_n && !h->full) {
             rbmnqs::SamplerShape best = h->shape;
             best_ms = -1;
             // one or two chains per warp, then the warps per block

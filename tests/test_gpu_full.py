@@ -166,3 +166,16 @@ def test_full_observables_are_weighted():
         ref = O.weighted_aggregate(lo, p, st["n_bins"])
         assert abs(vals[o, 0] + 1j * vals[o, 1] - ref["mean"]) < TOL64
         assert abs(vals[o, 2] - ref["stddev"]) < 1e-8 * max(1e-12, ref["stddev"])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_autotune_times_no_sweeps(precision):
+    """The launch-shape autotuner leaves the list of states alone: there are no
+    sweeps to time, and a sweep would record over it."""
+    _, _, s = make(model="kitaev", L=2, kind=1, alpha=2, precision=precision)
+    a = s.sample()
+    states, E = s.sample_configs(), s.samples(with_O=False)[0]
+    assert s.autotune(sweeps=2)[2] == 0
+    assert np.array_equal(s.sample_configs(), states)
+    b = s.sample()
+    assert a["energy"] == b["energy"] and np.array_equal(s.samples(with_O=False)[0], E)

@@ -40,7 +40,7 @@ bool plan_screen(const MachineDev& m, int fp64, int n_chains, int n_bonds, int m
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const int budget = smem_max - 8 * 1024;
-    screen::Layout L = screen::make_layout(m, n_bonds, 1, kBasicRows);
+    screen::Layout L = screen::make_layout(m, n_bonds, 1, kBasicRows, fp64);
     if (m.symmetric && (m.n + 1) * L.qs > 0xffff) return false;  // 16-bit row offsets
     const void* f = fp64 ? screen::pick_fp64(m, L.p_smem) : screen::pick_fp32(m, L.p_smem);
     if (!f) return false;
@@ -53,8 +53,8 @@ bool plan_screen(const MachineDev& m, int fp64, int n_chains, int n_bonds, int m
     wpb = std::min(wpb, (n_chains + sms - 1) / sms);
     if (max_wpb > 0) wpb = std::min(wpb, max_wpb);
     wpb = std::max(wpb, 1);
-    while (wpb > 1 && screen::make_layout(m, n_bonds, wpb, kBasicRows).total > budget) wpb--;
-    L = screen::make_layout(m, n_bonds, wpb, kBasicRows);
+    while (wpb > 1 && screen::make_layout(m, n_bonds, wpb, kBasicRows, fp64).total > budget) wpb--;
+    L = screen::make_layout(m, n_bonds, wpb, kBasicRows, fp64);
     if (L.total > budget) return false;
     if ((*err = ensure_dynamic_smem(f, L.total)) != cudaSuccess) return true;
     int per_sm = 0;
@@ -76,7 +76,7 @@ bool plan_screen(const MachineDev& m, int fp64, int n_chains, int n_bonds, int m
 
 cudaError_t launch_screen(const SamplerArgs& a0, int fp64, const SamplerShape& sh, cudaStream_t st) {
     SamplerArgs a = a0;
-    screen::Layout L = screen::make_layout(a.m, a.n_prop_bonds, sh.warps_per_block, sh.plan.p_budget);
+    screen::Layout L = screen::make_layout(a.m, a.n_prop_bonds, sh.warps_per_block, sh.plan.p_budget, fp64);
     const void* f = fp64 ? screen::pick_fp64(a.m, L.p_smem) : screen::pick_fp32(a.m, L.p_smem);
     if (!f || L.total != sh.smem || !a.m.P32) return cudaErrorInvalidValue;
     const cudaError_t e = ensure_dynamic_smem(f, L.total);

@@ -11,28 +11,50 @@
 //   ln|cosh theta'| - ln|cosh theta| = ln|1 + z p| - ln|1 + z| - 2 sigma_f Re W,
 // four FMA-pipe operations for the product, three for |1 + z p|^2, one to
 // multiply them up, one lg2 per four entries and no other transcendental.  When
-// |d - 0.5 ln u| exceeds what the two computations can differ by, the screen's
-// decision is the exact one; otherwise (about 1 % of the proposals) theta at the
-// start of the sweep is formed from its configuration in FP64, the sweep's
-// accepted flips are applied to it in FP32, in order, and decide_exact decides.
-// So chains, samples and counters are those of the exact sums, bit for bit.
+// |d - 0.5 ln u| exceeds a margin for what the two computations can differ by, the
+// screen decides; otherwise theta at the start of the sweep is formed from its
+// configuration in FP64, the sweep's accepted flips are applied to it in FP32, in
+// order, and decide_exact decides.
 //
 // Sessions in FP64 use the same screen; what it cannot tell is decided by the
-// ln|cosh| sums in FP64 (decide_fp64) on theta formed in FP64 from the current
-// configuration: the decisions of the FP64 sweep (sampler.cu run_chain) up to ties
-// of 1e-15.
+// ln|cosh| sums in FP64 (decide_fp64) on theta kept in FP64 in the same way.
 //
-// Error bound.  Away from the zeros of cosh both sums are good to a few 1e-5 (512
-// entries).  Near a zero the exact form loses digits: its |1 + w|^2 = 1 + |w|^2 +
-// 2 |w| cos carries the absolute error of the hardware cosine (2^-20.9, growing
-// with the argument) and exponential, so its ln is off by up to 1e-6 / |1 +
-// w|^2 per entry.  The margin is therefore m0 + coef (1 / min |1 + w|^2 at
-// theta' + 1 / min at theta), the minima over the entries, with m0 = 1e-3 + 2e-5
-// max |Re theta| and coef = 2e-6 + 5e-7 max |Im theta|, four times these errors,
-// max over all configurations of the machine (|b| + sum_f |W|).  z is refreshed
-// from theta every kRefresh sweeps: 1000 products of 1.2e-7 each stay below
-// 1e-5.  A machine that can reach |Re theta| > 40 leaves the FP32 range of z:
-// all its proposals take decide_exact.
+// The sums ln|1 + z| are kept as integers (2^-16 steps of lg2 a lane), so that the
+// difference of two of them is exact: in FP32 a sum of 1e4 is good to 1e-3.
+//
+// Margin, FP64 sessions.  A worst case, every rounding at its bound and all of one
+// sign: what the screen decides is what the sums in FP64 would, up to their own ties
+// of 1e-13.  In u = 2^-24 (set_margin):
+//  - z carries a relative error eps = u (6 max |Re theta| + 2 max |Im theta| + 24 + 3
+//    k) after k site flips: theta rounded, ex2 (2.5 u), the sine and cosine after
+//    their reduction (11 u; both measured over all floats), then per flip the
+//    rounding of p (u) and of a complex product with FMA (2 u; Jeannerod, Kornerup,
+//    Louvet, Muller, Math. Comp. 86, 2017).  An error common to z and w = z p moves
+//    d by eps |w - z| / (|1 + w| |1 + z|) per entry.  With a^2 and b^2 the largest 1 /
+//    |1 + z|^2 and 1 / |1 + w|^2 that is below |p - 1| (1 + a) b <= |p - 1| t with t =
+//    (1 + a^2) / 2 + b^2, and below 6 t however large p: the sum over the entries is S
+//    t eps, S the largest row's sum of min(exp(4 |W|) - 1, 6).
+//  - The products' own rounding of w, 3 u a site: |w / (1 + w)| <= 1 + b an entry.
+//  - The sums of ln|1 + z|: 2 u an entry for the squared moduli and their products, 2.6
+//    u + 2 u |lg2| a group (lg2, measured over all floats), the additions, and half a
+//    step a lane.
+// The first-order terms carry a factor 1.15 for the second order, which holds while
+// eps (1 + a) < 1/16; closer to a zero of cosh the margin is infinite, as where a
+// lane's sum leaves the integers' range (or is NaN).  It grows with the accepted
+// flips: z is refreshed from theta every four sweeps (FP32 sessions: eight).
+//
+// Margin, FP32 sessions.  The screen has to agree with the FP32 sums as they are
+// computed, and the worst cases of these (cosine and additions of |Re theta|, 1e-2
+// at 512 entries) exceed what they err by a hundredfold.  So the margin is an
+// estimate, m0 + coef (a^2 + b^2) with m0 = 8e-4 + 1e-4 max |Re theta| and coef = 2e-6
+// + 5e-7 max |Im theta|.  Over 5e7 proposals of machines of 384 and 512 entries
+// (weights of spread 0.005 to 0.1, hidden biases of either sign, near the zeros of
+// cosh, all entries of a unit equal) the largest difference was 0.29 of it, and the
+// screen's error against 64 bits below the sums' own.  A decision beyond it would
+// be one between two FP32 values of a tie, as the sums' decisions of ties are.
+//
+// A machine that can reach |Re theta| > 40 leaves the FP32 range of z: all its
+// proposals are decided by the sums.
 //
 // Layout: groups of KB consecutive hidden units with one symmetry index, lane l
 // owns the groups l + 32 j, entries in pairs (packed FP32x2).  Symmetric machines
@@ -47,13 +69,16 @@
 // 1.32 ms by the sums, 0.22 screened.
 #pragma once
 
+#include <type_traits>
+
 #include "eloc.cuh"
 #include "sweep_common.cuh"
 
 namespace rbmnqs {
 namespace screen {
 
-constexpr int kRefresh = 8;  // sweeps between refreshes of z
+// sweeps between refreshes of z
+__host__ __device__ constexpr int refresh_of(bool fp64) { return fp64 ? 4 : 8; }
 
 // A chain's state between the sweep loop and its services, in the warp's scratch
 // (z and z p of the last proposal: in local memory).  The loop keeps everything
@@ -63,15 +88,31 @@ constexpr int kRefresh = 8;  // sweeps between refreshes of z
 struct State {
     uint32_t start[4];  // configuration at the start of the sweep
     uint32_t sp[4];     // current configuration
-    float LS, lim;      // sum ln|1 + z|, coef / min |1 + z|^2
+    int LS;             // sum ln|1 + z|, in log_sum's steps
+    float inv;          // 1 / min |1 + z|^2
     int st, slot, np, applied;
     uint32_t prop, nacc;
+    int k;  // site flips since the refresh of z
     uint32_t code;      // the open proposal: sites, bond flag (bit 16), spins (bits 17, 18)
-    float lu, LSn, lim_n;
+    float lu;
+    int LSn;
+    float inv_n;
     int accept;
+    int sum_np;  // FP64 sessions: the sum of ln|cosh theta| after the sweep's first sum_np flips
+    double sum;
 };
-constexpr int kStateBytes = 96;
-static_assert(sizeof(State) <= kStateBytes, "state fits its slot");
+constexpr int kStateBytes = 112;
+
+// The margin of a proposal.  FP64: (fac (eps0 + eps1 k) + R1) t + R0 + R2 |LS| with
+// t = (1 + a^2) / 2 + b^2, k the site flips since the refresh of z and fac = 1, or fac2
+// for two sites; FP32: m0 + coef (a^2 + b^2).
+struct Margin {
+    float eps0, eps1, R0, R1, R2, fac2, mn_min;
+    float m0, coef;
+    // machine bounds (as uints, for atomicMax): max |Re theta|, max |Im theta|, S,
+    // max 4 |W|, max |sum_e Re W_fe + Re v|
+    unsigned bre, bim, S, xmax, smax;
+};
 
 // Hidden units per group: as the row loads can be widest for symmetric machines;
 // pairs for basic machines, whose lanes then read consecutive 16 bytes.
@@ -82,13 +123,14 @@ __host__ __device__ inline int group_width(const MachineDev& m) {
 
 // Shared-memory carve-up, the same arithmetic on host (sizing) and device.
 struct Layout {
-    int p, w, off, row, w64, base, site, bonds, lim, warp0, warp_bytes, total;
+    int p, w, off, row, w64, base, site, bonds, mar, warp0, warp_bytes, total;
+    int list;  // the sweep's accepted flips in a warp's scratch, behind theta
     int qs;    // row stride of p and W in shared memory (bytes)
     int ws64;  // row stride of the FP64 W (double2), shared or global
     int p_smem, w64_smem, bonds_smem;
 };
 // p_budget: bytes that the p table of a basic machine may take in shared memory
-__host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, int warps, int p_budget) {
+__host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, int warps, int p_budget, int fp64) {
     Layout L{};
     const int n = m.n, nh = m.nh, kb = group_width(m);
     const bool sym = m.symmetric != 0;
@@ -97,14 +139,15 @@ __host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, 
     L.w64_smem = sym && n * nh * 16 <= 32 * 1024;
     L.ws64 = L.w64_smem ? eloc::w64_stride(nh) : nh;
     L.bonds_smem = n_bonds * 8 <= 8 * 1024;
-    L.warp_bytes = kStateBytes + eloc::a16(m.T * 8) + eloc::a16(n * 4);
+    L.list = kStateBytes + eloc::a16(m.T * (fp64 ? 16 : 8));
+    L.warp_bytes = L.list + eloc::a16(n * 4);
     int at = 0;
     auto take = [&](int bytes) {
         const int o = at;
         at += eloc::a16(bytes);
         return o;
     };
-    // symmetric: two signs of n + 1 rows (row n: zero, read by groups beyond T)
+    // symmetric: two signs of n + 1 rows (row n, read by groups beyond T: p = 1)
     L.p = take(L.p_smem ? 2 * (n + 1) * L.qs : 0);
     L.w = take(L.p_smem ? (n + 1) * L.qs : 0);
     L.off = take(sym ? 2 * n * (m.S + 1) : 0);
@@ -113,27 +156,57 @@ __host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, 
     L.base = take(m.T * 16);
     L.site = take((n + 1) * 8);
     L.bonds = take(L.bonds_smem ? n_bonds * 8 : 0);
-    L.lim = take(8);
+    L.mar = take((int)sizeof(Margin));
     L.warp0 = at;
     L.total = at + warps * L.warp_bytes;
     return L;
 }
 
-__device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsigned char* smem) {
+// The margin's coefficients from the machine's bounds (see the top of the file).
+__device__ inline void set_margin(Margin& g, int n, int T, bool fp64) {
+    constexpr float u = 5.9604645e-8f, c = 1.15f;
+    const float bre = __uint_as_float(g.bre) * 1.001f, bim = __uint_as_float(g.bim) * 1.001f;
+    const float x = __uint_as_float(g.xmax) * 1.001f, sm = __uint_as_float(g.smax) * 1.001f;
+    if (fp64) {
+        // S of two rows: (e^x - 1)(e^y - 1) <= (their sum) max / 2, or both at their bound
+        const float t = (float)T, S = __uint_as_float(g.S) * 1.001f + 4.f * u * t;
+        const float e0 = 6.f * bre + 2.f * bim + 24.f, uu = u * 1.002f;
+        g.fac2 = 2.f * (1.f + fminf(0.5f * expm1f(x), 0.83f));
+        // common error of z; 3 u (1 + b) an entry and site: 1 + b <= 3 (1/2 + b^2)
+        g.eps0 = uu * c * (S * e0 + 9.f * t);
+        g.eps1 = uu * c * 3.f * S;
+        g.R0 = uu * (2840.f + 4.5f * t + 44.f * sm + 170.f);
+        g.R1 = uu * 3.68f * t;
+        g.R2 = uu * 10.5f;
+        const float eps = uu * (e0 + 3.f * (float)(refresh_of(true) * (n + 1) + 2));
+        g.mn_min = 400.f * eps * eps;
+    }
+    g.m0 = 8e-4f + 1e-4f * bre;
+    g.coef = 2e-6f + 5e-7f * bim;
+    if (!(bre < 40.f) || !(x < 84.f) || !(bim < 900.f)) g.m0 = g.R0 = __int_as_float(0x7f800000);
+}
+
+__device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsigned char* smem, bool fp64) {
     const MachineDev& m = a.m;
     const int tid = threadIdx.x, nt = blockDim.x;
     const int n = m.n, nh = m.nh, S = m.S, SP = S + 1;
     const bool sym = m.symmetric != 0;
     float* site = reinterpret_cast<float*>(smem + L.site);
-    unsigned* lim = reinterpret_cast<unsigned*>(smem + L.lim);
+    Margin* mar = reinterpret_cast<Margin*>(smem + L.mar);
     if (L.p_smem) {
         const int per = L.qs / 8;  // 8-byte slots a row, the padding zero
         float2* P = reinterpret_cast<float2*>(smem + L.p);
         float2* W = reinterpret_cast<float2*>(smem + L.w);
         for (int i = tid; i < 2 * (n + 1) * per; i += nt) {
             const int sg = i / ((n + 1) * per), r = i / per - sg * (n + 1), k = i % per;
-            P[i] = r < n && k < nh ? reinterpret_cast<const float2*>(m.P32)[(sg * n + r) * nh + k]
-                                   : make_float2(0.f, 0.f);
+            float2 v = make_float2(0.f, 0.f);
+            if (k < nh) {
+                if (r < n)
+                    v = reinterpret_cast<const float2*>(m.P32)[(sg * n + r) * nh + k];
+                else if (sym)  // pairs of parts, or one entry's
+                    v = (nh & 1) ? make_float2(1.f, 0.f) : ((k & 1) ? v : make_float2(1.f, 1.f));
+            }
+            P[i] = v;
         }
         for (int i = tid; i < (n + 1) * per; i += nt) {
             const int r = i / per, k = i % per;
@@ -158,10 +231,10 @@ __device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsign
         for (int i = tid; i < a.n_prop_bonds; i += nt) b[i] = a.prop_bonds[i];
     }
     // Re v (bias term of the exact sum) beside sum_e Re W_fe + Re v
-    if (tid < 2) lim[tid] = 0;
+    if (tid == 0) mar->bre = mar->bim = mar->S = mar->xmax = mar->smax = 0;
     __syncthreads();
     const double2* W64 = L.w64_smem ? reinterpret_cast<const double2*>(smem + L.w64) : m.W64;
-    // theta of the all-up configuration, and the bounds |b| + sum_f |W|
+    // theta of the all-up configuration and the bounds |b| + sum_f |W|
     double2* base = reinterpret_cast<double2*>(smem + L.base);
     for (int t = tid; t < m.T; t += nt) {
         const int k = t % nh, s = t / nh;
@@ -176,30 +249,41 @@ __device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsign
         }
         base[t] = acc;
         // non-finite weights give bounds above any limit
-        atomicMax(&lim[0], __float_as_uint(bx == bx ? bx : 1e30f));
-        atomicMax(&lim[1], __float_as_uint(by == by ? by : 1e30f));
+        atomicMax(&mar->bre, __float_as_uint(bx == bx ? bx : 1e30f));
+        atomicMax(&mar->bim, __float_as_uint(by == by ? by : 1e30f));
     }
     for (int f = tid >> 5; f <= n; f += nt >> 5) {  // a warp per site
         double acc = 0;
+        float S = 0.f, xm = 0.f;
         if (f < n)
-            for (int t = tid & 31; t < m.T; t += 32)
-                acc += W64[(sym ? (int)smem[L.row + f * SP + t / nh] : f) * L.ws64 + t % nh].x;
+            for (int t = tid & 31; t < m.T; t += 32) {
+                const double2 w = W64[(sym ? (int)smem[L.row + f * SP + t / nh] : f) * L.ws64 + t % nh];
+                acc += w.x;
+                const float wx = (float)w.x, wy = (float)w.y, x = 4.f * sqrtf(wx * wx + wy * wy);
+                S += fminf(ex2_ftz(1.442696f * x) - 1.f, 6.f);  // NaN: bre, bim
+                xm = fmaxf(xm, x);
+            }
         acc = warp_sum(acc);
+        S = warp_sum(S);
+        xm = warp_max(xm);
         if ((tid & 31) == 0) {
             const float v = f < n ? (float)m.vb[f % m.n_vb].x : 0.f;
+            const float s = f < n ? (float)(acc + m.vb[f % m.n_vb].x) : 0.f;
             site[2 * f] = v;
-            site[2 * f + 1] = f < n ? (float)(acc + m.vb[f % m.n_vb].x) : 0.f;
+            site[2 * f + 1] = s;
+            const float sm = fabsf(s) + fabsf(v);
+            atomicMax(&mar->S, __float_as_uint(fmaxf(S, 0.f)));
+            atomicMax(&mar->xmax, __float_as_uint(xm));
+            atomicMax(&mar->smax, __float_as_uint(sm == sm ? sm : 1e30f));
         }
     }
     __syncthreads();
+    if (tid == 0) set_margin(*mar, n, m.T, fp64);
+    __syncthreads();
 }
 
-// A warp's scratch: the configuration at the start of the sweep (16 bytes),
-// theta [T] in FP32, the sweep's accepted flips.
-__device__ __forceinline__ float2* theta_scratch(unsigned char* wscr) { return reinterpret_cast<float2*>(wscr + 16); }
-
-// One chain.  wscr: the warp's scratch (theta [T] FP32, the sweep's accepted
-// flips [n]).  PS: p and W rows in shared memory (always for symmetric machines).
+// One chain.  wscr: the warp's scratch (state, theta [T] in the session's precision,
+// the sweep's accepted flips [n]).  PS: p and W rows in shared memory (always for symmetric machines).
 template <int KB, int NG, bool SYM, bool PS, bool F64>
 __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L, unsigned char* smem,
                                           unsigned char* wscr, int chain, int lane) {
@@ -210,8 +294,9 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
     const uint2 key = make_uint2((uint32_t)a.seed, (uint32_t)(a.seed >> 32));
     const uint32_t epoch = a.ctl[0];
     State* S = reinterpret_cast<State*>(wscr);
-    float2* th = reinterpret_cast<float2*>(wscr + kStateBytes);
-    uint32_t* plist = reinterpret_cast<uint32_t*>(wscr + kStateBytes + eloc::a16(T * 8));
+    using TH = std::conditional_t<F64, double2, float2>;
+    TH* th = reinterpret_cast<TH*>(wscr + kStateBytes);
+    uint32_t* plist = reinterpret_cast<uint32_t*>(wscr + L.list);
     {
         uint32_t sp[4];
         chain_start(a, chain, key, epoch, sp);
@@ -242,8 +327,8 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
         ko[j] = 8u * (uint32_t)(SYM ? (ok ? (g % NGK) * KB : 0) : (ok ? g * KB : 0));
     }
 
-    // theta of configuration S->start (FP64, down spins in increasing order),
-    // rounded to FP32 into the scratch, two groups at a time
+    // theta of configuration S->start (FP64, down spins in increasing order)
+    // into the scratch, two groups at a time
     auto theta_of = [&]() {
         constexpr int NJ = NG >= 2 ? 2 : 1;
 #pragma unroll 1
@@ -281,8 +366,12 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                 const int g = lane + 32 * (j0 + j);
                 if (g < G)
 #pragma unroll
-                    for (int i = 0; i < KB; i++)
-                        th[KB * g + i] = make_float2((float)acc[KB * j + i].x, (float)acc[KB * j + i].y);
+                    for (int i = 0; i < KB; i++) {
+                        if constexpr (F64)
+                            th[KB * g + i] = acc[KB * j + i];
+                        else
+                            th[KB * g + i] = make_float2((float)acc[KB * j + i].x, (float)acc[KB * j + i].y);
+                    }
             }
         }
         __syncwarp();
@@ -298,45 +387,64 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             return __ldg(m.W32 + f * nh + t);
         }
     };
-    // The FP64 sessions' decision: u < |psi'/psi|^2 by the ln|cosh| sums in FP64,
-    // theta formed from the current configuration.
-    auto decide_fp64 = [&](uint32_t code, uint32_t prop) -> bool {
+    // The FP64 sessions' decision: u < |psi'/psi|^2 by the ln|cosh| sums in FP64, after
+    // the accepted flips from `applied` on have been applied to theta in the
+    // scratch.  The sum at theta is kept for the next open proposal (S->sum, of
+    // the sweep's first S->sum_np flips).
+    auto decide_fp64 = [&](uint32_t code, uint32_t prop, int applied, int np) -> bool {
+        auto w64 = [&](int f, int q, int k) -> double2 {
+            return W64[(SYM ? (int)rows[f * SP + q] : f) * L.ws64 + k];
+        };
         const int f0 = code & 255u, f1 = (code >> 8) & 255u;
-        const bool bond = (code >> 16) & 1u;
+        const bool bond = (code >> 16) & 1u, kept = S->sum_np == np;
         const double g0 = (code >> 17) & 1u ? 2.0 : -2.0, g1 = (code >> 18) & 1u ? 2.0 : -2.0;
-        double d = 0;
+        double sx = 0, sy = 0;
 #pragma unroll 1
         for (int t = lane; t < T; t += 32) {
             const int q = SYM ? t / nh : 0, k = SYM ? t - q * nh : t;
-            double2 x = base[t];
+            double2 x;
+            if constexpr (F64) x = th[t];
 #pragma unroll 1
-            for (int wd = 0; wd < 4; wd++) {
-                uint32_t bits = S->sp[wd];
-                while (bits) {
-                    const int f = 32 * wd + __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const double2 w = W64[(SYM ? (int)rows[f * SP + q] : f) * L.ws64 + k];
-                    x.x = fma(-2.0, w.x, x.x);
-                    x.y = fma(-2.0, w.y, x.y);
+            for (int i = applied; i < np; i++) {
+                const uint32_t c = plist[i];
+                const double h0 = (c >> 17) & 1u ? 2.0 : -2.0, h1 = (c >> 18) & 1u ? 2.0 : -2.0;
+                double2 w = w64(c & 255u, q, k);
+                x.x = fma(h0, w.x, x.x);
+                x.y = fma(h0, w.y, x.y);
+                if ((c >> 16) & 1u) {
+                    w = w64((c >> 8) & 255u, q, k);
+                    x.x = fma(h1, w.x, x.x);
+                    x.y = fma(h1, w.y, x.y);
                 }
             }
-            double2 w = W64[(SYM ? (int)rows[f0 * SP + q] : f0) * L.ws64 + k];
+            if constexpr (F64) th[t] = x;
+            if (!kept) sx += lnc_re<double>(x.x, x.y);
+            double2 w = w64(f0, q, k);
             double2 y = make_double2(fma(g0, w.x, x.x), fma(g0, w.y, x.y));
             if (bond) {
-                w = W64[(SYM ? (int)rows[f1 * SP + q] : f1) * L.ws64 + k];
+                w = w64(f1, q, k);
                 y = make_double2(fma(g1, w.x, y.x), fma(g1, w.y, y.y));
             }
-            d += lnc_re<double>(y.x, y.y) - lnc_re<double>(x.x, x.y);
+            sy += lnc_re<double>(y.x, y.y);
         }
-        d = warp_sum(d) + g0 * m.vb[f0 % m.n_vb].x;
+        sx = kept ? S->sum : warp_sum(sx);
+        sy = warp_sum(sy);
+        double d = sy - sx + g0 * m.vb[f0 % m.n_vb].x;
         if (bond) d += g1 * m.vb[f1 % m.n_vb].x;
         const uint4 r = philox4x32(make_uint4(prop, epoch, (uint32_t)chain, 0), key);
-        return unit24<double>(r.z) < exp(2.0 * d);
+        const bool accept = unit24<double>(r.z) < exp(2.0 * d);
+        __syncwarp();
+        if (lane == 0) {
+            S->sum = accept ? sy : sx;
+            S->sum_np = accept ? np + 1 : np;
+        }
+        return accept;
     };
     // d of a proposal (code: sites, bond flag in bit 16, spins of the sites in
     // bits 17 and 18) by the ln|cosh| sums of theta and theta' over the entries
     // lane + 32 e, in the arithmetic of lnc_sweep_sum and sweep_sum, after the
     // accepted flips from `applied` on have been applied to theta in the scratch
+    float2* th32 = reinterpret_cast<float2*>(th);
     auto decide_exact = [&](uint32_t code, int applied, int np) -> float {
 #pragma unroll 1
         for (; applied < np; applied++) {
@@ -346,9 +454,9 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             const bool two = (c >> 16) & 1u;
 #pragma unroll 4
             for (int t = lane; t < T; t += 32) {
-                float2 v = __ffma2_rn(make_float2(h0, h0), wrow(q0, t), th[t]);
+                float2 v = __ffma2_rn(make_float2(h0, h0), wrow(q0, t), th32[t]);
                 if (two) v = __ffma2_rn(make_float2(h1, h1), wrow(q1, t), v);
-                th[t] = v;
+                th32[t] = v;
             }
         }
         const int f0 = code & 255u, f1 = (code >> 8) & 255u;
@@ -364,7 +472,7 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                 const int t = lane + 32 * (e0 + q);
                 float2 x = make_float2(0.f, 0.f), y = x;
                 if (t < T) {
-                    x = th[t];
+                    x = th32[t];
                     y = __ffma2_rn(make_float2(g0, g0), wrow(f0, t), x);
                     if (bond) y = __ffma2_rn(make_float2(g1, g1), wrow(f1, t), y);
                 }
@@ -386,8 +494,11 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
     };
 
     // squared moduli of 1 + z over the lane's entries: the sum of their lg2 in
-    // 2^-16 steps over the warp (times ln 2 / 2: sum ln|1 + z|) and their minimum
-    auto log_sum = [&](const float2 (&xr)[NP], const float2 (&xi)[NP], float& mn) -> float {
+    // 2^-16 steps over the warp (times ln 2 / 2: sum ln|1 + z|) and one over their
+    // minimum
+    const Margin& mar = *reinterpret_cast<const Margin*>(smem + L.mar);
+    constexpr float kStep = 0.346573590279972655f / 65536.f;
+    auto log_sum = [&](const float2 (&xr)[NP], const float2 (&xi)[NP], float& inv) -> int {
         float lg = 0.f, lo = 1e30f;
         const float2 one = make_float2(1.f, 1.f);
 #pragma unroll
@@ -403,14 +514,20 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             }
             lg += lg2_ftz(q.x * q.y);
         }
-        // out of range (or NaN): a minimum of 0, an infinite margin
-        mn = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(fabsf(lg) < 1000.f ? lo : 0.f)));
-        return (float)__reduce_add_sync(kFull, __float2int_rn(lg * 65536.f)) * (0.346573590279972655f / 65536.f);
+        // outside +-511 (or NaN): a minimum of 0, an infinite margin.  Inside, two
+        // totals differ by less than 2^31 steps
+        const float mn = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(fabsf(lg) < 511.f ? lo : 0.f)));
+        inv = __fdividef(1.f, mn);
+        if constexpr (F64)
+            if (!(mn > mar.mn_min)) inv = __int_as_float(0x7f800000);
+        return __reduce_add_sync(kFull, __float2int_rn(lg * 65536.f));
     };
-    const float bre = __uint_as_float(reinterpret_cast<const unsigned*>(smem + L.lim)[0]);
-    const float bim = __uint_as_float(reinterpret_cast<const unsigned*>(smem + L.lim)[1]);
-    const float m0 = bre > 40.f ? __int_as_float(0x7f800000) : 1e-3f + 2e-5f * bre;
-    const float coef = 2e-6f + 5e-7f * bim;
+    const float m0 = mar.m0, coef = mar.coef;
+    // FP64 margin's part that accepted proposals change
+    auto margin = [&](int LS, int k, float& eps) -> float {
+        eps = fmaf(mar.eps1, (float)k, mar.eps0);
+        return fmaf(mar.R2 * kStep, fabsf((float)LS), mar.R0);
+    };
     // w = x p(f, spin sg)
     auto times_p = [&](int f, int sg, const float2 (&xr)[NP], const float2 (&xi)[NP], float2 (&wr)[NP],
                        float2 (&wi)[NP]) {
@@ -466,9 +583,10 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             const int st = S->st;
             if (lane < 4) S->start[lane] = S->sp[lane];
             __syncwarp();
-            if (st == 0 && a.theta_in && a.plan.lane_rows) {
+            if (!F64 && st == 0 && a.theta_in && a.plan.lane_rows) {
                 const float2* src = a.theta_in + (size_t)chain * 32 * a.plan.lane_entries;
-                for (int t = lane; t < T; t += 32) th[t] = src[t];
+                if constexpr (!F64)
+                    for (int t = lane; t < T; t += 32) th[t] = src[t];
                 __syncwarp();
             } else {
                 theta_of();
@@ -480,9 +598,11 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                 const int g = lane + 32 * j;
 #pragma unroll
                 for (int i = 0; i < KB; i++) {
-                    float2 z = make_float2(0.f, 0.f);
+                    // beyond T: 1 (p = 1), whose |1 + z|^2 is never the smallest for
+                    // long; basic machines 0, since their p is another group's
+                    float2 z = make_float2(SYM ? 1.f : 0.f, 0.f);
                     if (g < G) {
-                        const float2 t = th[KB * g + i];
+                        const float2 t = make_float2((float)th[KB * g + i].x, (float)th[KB * g + i].y);
                         const float r = ex2_ftz(t.x * -2.88539008177792681f);
                         float s, c;
                         sincos_r(2.f * t.y, &s, &c);
@@ -498,8 +618,8 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                     }
                 }
             }
-            float mn;
-            const float ls = log_sum(zr, zi, mn);
+            float inv;
+            const int ls = log_sum(zr, zi, inv);
 #pragma unroll
             for (int p = 0; p < NP; p++) {
                 hold[4 * p] = zr[p].x;
@@ -509,24 +629,27 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             }
             if (lane == 0) {
                 S->LS = ls;
-                S->lim = __fdividef(coef, mn);
+                S->inv = inv;
+                S->k = 0;
                 S->applied = 0;
+                S->sum_np = -1;
                 S->accept = 0;
             }
             __syncwarp();
         } else {
             const int np = S->np;
-            bool accept;
-            if constexpr (F64) {
-                accept = decide_fp64(S->code, S->prop - 1);
-            } else {
-                int applied = S->applied;
-                if (applied < 0) {
-                    theta_of();
-                    applied = 0;
-                }
-                accept = S->lu < decide_exact(S->code, applied, np);
+            int applied = S->applied;
+            if (applied < 0) {
+                theta_of();
+                applied = 0;
+                if (lane == 0) S->sum_np = -1;
+                __syncwarp();
             }
+            bool accept;
+            if constexpr (F64)
+                accept = decide_fp64(S->code, S->prop - 1, applied, np);
+            else
+                accept = S->lu < decide_exact(S->code, applied, np);
             __syncwarp();
             if (lane == 0) {
                 S->applied = np;
@@ -534,10 +657,11 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                 if (accept) {
                     const uint32_t c = S->code;
                     S->LS = S->LSn;
-                    S->lim = S->lim_n;
-                    if constexpr (!F64) plist[np] = c;
+                    S->inv = S->inv_n;
+                    plist[np] = c;
                     S->np = np + 1;
                     S->nacc++;
+                    S->k += (c >> 16) & 1u ? 2 : 1;
                     S->sp[(c & 255u) >> 5] ^= 1u << (c & 31u);
                     if ((c >> 16) & 1u) S->sp[((c >> 8) & 255u) >> 5] ^= 1u << ((c >> 8) & 31u);
                 }
@@ -555,10 +679,13 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             }
         }
         const uint32_t spa = smem_addr(S->sp);  // the configuration stays in the scratch
-        float LS = S->LS, lim_cur = S->lim;
+        int LS = S->LS;
+        float inv = S->inv;
         int st = S->st, slot = S->slot, np = S->np, applied = S->applied;
         uint32_t prop = S->prop, nacc = S->nacc, pcode = 0;
-        float plu = 0.f;
+        float plu = 0.f, eps = 0.f, rest = 0.f;
+        int k = S->k;
+        if constexpr (F64) rest = margin(LS, k, eps);
         auto draw = [&]() {  // this lane's proposal of the batch of 32
             const uint4 r = philox4x32(make_uint4((prop & ~31u) + lane, epoch, (uint32_t)chain, 0), key);
             uint32_t f0, f1, bond;
@@ -587,7 +714,7 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                 st++;
                 slot = np = 0;
                 applied = -1;
-                if (st == total || st % kRefresh == 0) break;
+                if (st == total || st % refresh_of(F64) == 0) break;
                 if (lane < 4) S->start[lane] = S->sp[lane];
             }
             if ((prop & 31u) == 0) draw();
@@ -605,12 +732,16 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             float2 wr[NP], wi[NP];
             times_p(f0, b0, zr, zi, wr, wi);
             if (bond) times_p(f1, b1, wr, wi, wr, wi);
-            float mn;
-            const float LSn = log_sum(wr, wi, mn);
-            const float lim_new = __fdividef(coef, mn);
-            const float D = fmaf(g1, lds_f2(sa + 8u * f1).y, fmaf(g0, lds_f2(sa + 8u * f0).y, LSn - LS));
+            float inv_n;
+            const int LSn = log_sum(wr, wi, inv_n);
+            const float D = fmaf(g1, lds_f2(sa + 8u * f1).y, fmaf(g0, lds_f2(sa + 8u * f0).y, (float)(int)((unsigned)LSn - (unsigned)LS) * kStep));
             const uint32_t full = code | (b0 << 17) | (b1 << 18);
-            if (!(fabsf(D - lu) > m0 + lim_new + lim_cur)) {
+            float mg;
+            if constexpr (F64)
+                mg = fmaf(fmaf(bond ? mar.fac2 : 1.f, eps, mar.R1), fmaf(0.5f, inv + 1.f, inv_n), rest);
+            else
+                mg = fmaf(coef, inv_n + inv, m0);
+            if (!(fabsf(D - lu) > mg)) {
 #pragma unroll
                 for (int p = 0; p < NP; p++) {
                     hold[4 * (NP + p)] = wr[p].x;
@@ -622,7 +753,7 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                     S->code = full;
                     S->lu = lu;
                     S->LSn = LSn;
-                    S->lim_n = lim_new;
+                    S->inv_n = inv_n;
                 }
                 open = true;
                 break;
@@ -634,15 +765,19 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
                     zi[p] = wi[p];
                 }
                 LS = LSn;
-                lim_cur = lim_new;
+                inv = inv_n;
                 if (lane == 0) {
-                    if constexpr (!F64) plist[np] = full;
+                    plist[np] = full;
                     S->sp[f0 >> 5] ^= 1u << (f0 & 31);
                     if (bond) S->sp[f1 >> 5] ^= 1u << (f1 & 31);
                 }
                 __syncwarp();
                 np++;
                 nacc++;
+                if constexpr (F64) {
+                    k += bond ? 2 : 1;
+                    rest = margin(LS, k, eps);
+                }
             }
         }
         // ---- back to the state
@@ -657,13 +792,14 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
         }
         if (lane == 0) {
             S->LS = LS;
-            S->lim = lim_cur;
+            S->inv = inv;
             S->st = st;
             S->slot = slot;
             S->np = np;
             S->applied = applied;
             S->prop = prop;
             S->nacc = nacc;
+            S->k = k;
         }
         __syncwarp();
         if (!open && st == total && !a.theta_out) break;
@@ -672,7 +808,7 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
         // FP32 theta of the final configuration, zero beyond T
         const int TP = 32 * a.plan.lane_entries;
         float2* dst = a.theta_out + (size_t)chain * TP;
-        for (int t = lane; t < TP; t += 32) dst[t] = t < T ? th[t] : make_float2(0.f, 0.f);
+        for (int t = lane; t < TP; t += 32) dst[t] = t < T ? th32[t] : make_float2(0.f, 0.f);
     }
     const uint32_t sp[4] = {S->sp[0], S->sp[1], S->sp[2], S->sp[3]};
     chain_finish(a, chain, lane, sp, S->nacc, S->prop);
@@ -686,7 +822,7 @@ __host__ __device__ constexpr int max_threads(int E) { return E >= 16 ? 512 : (E
 template <int KB, int NG, bool SYM, bool PS, bool F64>
 __global__ void __launch_bounds__(max_threads(KB* NG), 1) screen_kernel(const SamplerArgs a, const Layout L) {
     extern __shared__ __align__(16) unsigned char smem[];
-    load_tables(a, L, smem);
+    load_tables(a, L, smem, F64);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_warps = (blockDim.x >> 5) * gridDim.x;
     // consecutive chains on different SMs

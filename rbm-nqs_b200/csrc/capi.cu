@@ -319,6 +319,7 @@ struct rbmnqs_handle {
     DevBuf<double2> params, vb, hb, W64, x;
     DevBuf<float2> W32;
     DevBuf<float> P32;  // exp(+-4 W) for the screened sweep
+    DevBuf<int> screen_off;
     DevBuf<uint8_t> perm, inv, orbit;
     DevBuf<uint8_t> wrank;  // row order of W in the FP32 evaluation kernel (symmetric machines)
     DevBuf<rbmnqs::OpDev> ops;
@@ -530,6 +531,7 @@ struct rbmnqs_handle {
         a.seed = cfg.seed;
         a.spins = spins.p;
         a.samples = samples.p;
+        a.screen_off = screen_off.p;
         a.n_acc = nacc.p;
         a.n_prop = nprop.p;
         return a;
@@ -1360,6 +1362,7 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
            "sampler plan");
         if (h->shape.plan.screen && !h->full) {
             h->P32.alloc((size_t)4 * n * nh);
+            h->screen_off.alloc(1);
             // the factors of the zero weights
             ck(rbmnqs::launch_unpack(h->params.p, n, h->n_vb, nh, h->vb.p, h->hb.p, h->W64.p, h->W32.p, h->P32.p, h->st),
                "unpack");

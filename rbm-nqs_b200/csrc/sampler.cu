@@ -1435,6 +1435,7 @@ template <int E, typename R, int FAST, bool PF>
 __global__ void __launch_bounds__(FAST == 2 ? MaxThreads<E, PF>::gather
                                             : (FAST == 3 ? MaxThreads<E, PF>::pair : MaxThreads<E, PF>::v),
                                   1) sampler_kernel(const SamplerArgs a) {
+    if (a.gate && !*a.gate) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int fp64 = sizeof(R) == 8;
     Smem sm = carve(smem, a.m, fp64, a.plan, a.n_prop_bonds, sweep_warp_bytes(a.m.T, sizeof(R), PF));
@@ -2258,8 +2259,13 @@ cudaError_t plan_sampler(const MachineDev& m, int fp64, int n_chains, int n_bond
                          int pair_mode, bool screen) {
     cudaError_t err = cudaSuccess;
     if (m.pf.n == 0 && (fp64 || (screen && pair_mode != 1)) &&
-        plan_screen(m, fp64, n_chains, n_bonds, max_wpb, out, &err))
+        plan_screen(m, fp64, n_chains, n_bonds, max_wpb, out, &err)) {
+        if (err != cudaSuccess) return err;
+        SamplerShape ex{};
+        err = plan_sampler_impl(m, fp64, n_chains, n_bonds, &ex, max_wpb, 0);
+        out->exact = ex;
         return err;
+    }
     return plan_sampler_impl(m, fp64, n_chains, n_bonds, out, max_wpb, pair_mode);
 }
 
@@ -2288,14 +2294,21 @@ bool sampler_writes_theta(const MachineDev& m, int fp64, const SamplerShape& sh)
 cudaError_t launch_sampler(const SamplerArgs& a0, int fp64, const SamplerShape& sh, cudaStream_t st) {
     SamplerArgs a = a0;
     a.plan = sh.plan;
-    if (sh.plan.screen) return launch_screen(a, fp64, sh, st);
+    SweepShape ex = sh;
+    if (sh.plan.screen) {
+        const cudaError_t e = launch_screen(a, fp64, sh, st);
+        if (e != cudaSuccess) return e;
+        ex = sh.exact;
+        a.plan = ex.plan;
+        a.gate = a.screen_off;
+    }
     const int E = elements_per_lane(a.m.T);
-    const void* fn = pick_sampler(E, fp64, sh.plan.use_u, a.m.pf.n > 0, sh.plan.gather, sh.plan.pair);
+    const void* fn = pick_sampler(E, fp64, ex.plan.use_u, a.m.pf.n > 0, ex.plan.gather, ex.plan.pair);
     if (!fn) return cudaErrorInvalidValue;
-    const cudaError_t e = ensure_dynamic_smem(fn, sh.smem);
+    const cudaError_t e = ensure_dynamic_smem(fn, ex.smem);
     if (e != cudaSuccess) return e;
     void* args[] = {&a};
-    return cudaLaunchKernel(fn, dim3(sh.blocks), dim3(32 * sh.warps_per_block), args, sh.smem, st);
+    return cudaLaunchKernel(fn, dim3(ex.blocks), dim3(32 * ex.warps_per_block), args, ex.smem, st);
 }
 
 template <int E, typename R, bool PF>

@@ -101,6 +101,10 @@ struct SamplerArgs {
     // (learned moves between sweep launches); used by the lane-ordered
     // gather path, the others recompute; null: recomputed
     const float2* theta_in = nullptr;
+    // set by the screened sweep when it leaves the whole launch to the sums'
+    // kernel, which is launched behind it and runs only then (gate)
+    int* screen_off = nullptr;
+    const int* gate = nullptr;
 };
 
 // The Hamiltonian regrouped by transition for the FP32 evaluation kernel
@@ -201,11 +205,14 @@ int eval_smem_bytes(const MachineDev& m, int fp64, int warps, const SmemPlan& pl
 // Plan + launch shape of the sampler for this machine and chain count:
 // one persistent block per SM with enough warps to hold every chain when
 // registers allow.
-struct SamplerShape {
+struct SweepShape {
     SmemPlan plan;
     int warps_per_block;
     int blocks;
     int smem;
+};
+struct SamplerShape : SweepShape {
+    SweepShape exact;  // screened sweep: the sums' kernel behind it
 };
 // max_wpb > 0 caps the warps per block (launch-shape autotuning); pair_mode
 // 1 asks for two chains per warp where the table path allows it (else, and

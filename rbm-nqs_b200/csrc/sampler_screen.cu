@@ -78,7 +78,7 @@ cudaError_t launch_screen(const SamplerArgs& a0, int fp64, const SamplerShape& s
     SamplerArgs a = a0;
     screen::Layout L = screen::make_layout(a.m, a.n_prop_bonds, sh.warps_per_block, sh.plan.p_budget, fp64);
     const void* f = fp64 ? screen::pick_fp64(a.m, L.p_smem) : screen::pick_fp32(a.m, L.p_smem);
-    if (!f || L.total != sh.smem || !a.m.P32) return cudaErrorInvalidValue;
+    if (!f || L.total != sh.smem || !a.m.P32 || !a.screen_off) return cudaErrorInvalidValue;
     const cudaError_t e = ensure_dynamic_smem(f, L.total);
     if (e != cudaSuccess) return e;
     void* args[] = {&a, &L};

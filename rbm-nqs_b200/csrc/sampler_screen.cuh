@@ -53,8 +53,12 @@
 // screen's error against 64 bits below the sums' own.  A decision beyond it would
 // be one between two FP32 values of a tie, as the sums' decisions of ties are.
 //
-// A machine that can reach |Re theta| > 40 leaves the FP32 range of z: all its
-// proposals are decided by the sums.
+// Weights that leave too many proposals open (kOff: the FP64 margin at mean counts
+// and |1 + z| = 1), that reach |Re theta| > 40, that mostly overflow a product of four
+// |1 + z|^2 (a sum of -Re theta of 22; 512 entries of 128 spins: spread of the weights
+// 0.2 0.2 % of the proposals, 0.25 48 %, 0.3 94 %), or that FP32 factors do not hold, turn the launch over
+// to the sums' kernel (sampler.cu), which is launched behind this one and returns at
+// once otherwise.
 //
 // Layout: groups of KB consecutive hidden units with one symmetry index, lane l
 // owns the groups l + 32 j, entries in pairs (packed FP32x2).  Symmetric machines
@@ -109,10 +113,13 @@ constexpr int kStateBytes = 112;
 struct Margin {
     float eps0, eps1, R0, R1, R2, fac2, mn_min;
     float m0, coef;
+    int off;  // the launch is left to the sums' kernel
     // machine bounds (as uints, for atomicMax): max |Re theta|, max |Im theta|, S,
-    // max 4 |W|, max |sum_e Re W_fe + Re v|
-    unsigned bre, bim, S, xmax, smax;
+    // max 4 |W|, max |sum_e Re W_fe + Re v|, and what -Re theta of four entries may add
+    // up to: their hidden biases' part and eight times theta's spread
+    unsigned bre, bim, S, xmax, smax, sat;
 };
+constexpr float kOff = 0.3f, kSat32 = 21.f, kSat64 = 30.f;
 
 // Hidden units per group: as the row loads can be widest for symmetric machines;
 // pairs for basic machines, whose lanes then read consecutive 16 bytes.
@@ -163,10 +170,12 @@ __host__ __device__ inline Layout make_layout(const MachineDev& m, int n_bonds, 
 }
 
 // The margin's coefficients from the machine's bounds (see the top of the file).
-__device__ inline void set_margin(Margin& g, int n, int T, bool fp64) {
+// E: entries per lane; with two, the products are of two.
+__device__ inline void set_margin(Margin& g, int n, int T, int E, bool fp64, bool bonds) {
     constexpr float u = 5.9604645e-8f, c = 1.15f;
     const float bre = __uint_as_float(g.bre) * 1.001f, bim = __uint_as_float(g.bim) * 1.001f;
     const float x = __uint_as_float(g.xmax) * 1.001f, sm = __uint_as_float(g.smax) * 1.001f;
+    float typ = 0.f;
     if (fp64) {
         // S of two rows: (e^x - 1)(e^y - 1) <= (their sum) max / 2, or both at their bound
         const float t = (float)T, S = __uint_as_float(g.S) * 1.001f + 4.f * u * t;
@@ -180,10 +189,12 @@ __device__ inline void set_margin(Margin& g, int n, int T, bool fp64) {
         g.R2 = uu * 10.5f;
         const float eps = uu * (e0 + 3.f * (float)(refresh_of(true) * (n + 1) + 2));
         g.mn_min = 400.f * eps * eps;
+        typ = g.R0 + g.R2 * t + 2.f * ((bonds ? g.fac2 : 1.f) * (g.eps0 + g.eps1 * n) + g.R1);
     }
     g.m0 = 8e-4f + 1e-4f * bre;
     g.coef = 2e-6f + 5e-7f * bim;
-    if (!(bre < 40.f) || !(x < 84.f) || !(bim < 900.f)) g.m0 = g.R0 = __int_as_float(0x7f800000);
+    g.off = !(typ < kOff) || !(bre < 40.f) || !(x < 84.f) || !(bim < 900.f) ||
+            !(__uint_as_float(g.sat) < (fp64 ? kSat64 : kSat32) * (E > 2 ? 1.f : 2.f));
 }
 
 __device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsigned char* smem, bool fp64) {
@@ -231,26 +242,40 @@ __device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsign
         for (int i = tid; i < a.n_prop_bonds; i += nt) b[i] = a.prop_bonds[i];
     }
     // Re v (bias term of the exact sum) beside sum_e Re W_fe + Re v
-    if (tid == 0) mar->bre = mar->bim = mar->S = mar->xmax = mar->smax = 0;
+    if (tid == 0) mar->bre = mar->bim = mar->S = mar->xmax = mar->smax = mar->sat = 0;
     __syncthreads();
     const double2* W64 = L.w64_smem ? reinterpret_cast<const double2*>(smem + L.w64) : m.W64;
-    // theta of the all-up configuration and the bounds |b| + sum_f |W|
+    // theta of the all-up configuration, the bounds |b| + sum_f |W|, and per group
+    // of hidden units sum -Re b and theta's variance
     double2* base = reinterpret_cast<double2*>(smem + L.base);
-    for (int t = tid; t < m.T; t += nt) {
-        const int k = t % nh, s = t / nh;
-        double2 acc = m.hb[k];
-        float bx = fabsf((float)acc.x), by = fabsf((float)acc.y);
-        for (int f = 0; f < n; f++) {
-            const double2 w = W64[(sym ? (int)smem[L.row + f * SP + s] : f) * L.ws64 + k];
-            acc.x += w.x;
-            acc.y += w.y;
-            bx += fabsf((float)w.x);
-            by += fabsf((float)w.y);
+    const int kb = group_width(m);
+    for (int t0 = 0; t0 < m.T; t0 += nt) {
+        const int t = t0 + tid, k = t % nh, s = t / nh;
+        float b = 0.f, v = 0.f;
+        if (t < m.T) {
+            double2 acc = m.hb[k];
+            float bx = fabsf((float)acc.x), by = fabsf((float)acc.y);
+            b = fmaxf(-(float)acc.x, 0.f);
+            for (int f = 0; f < n; f++) {
+                const double2 w = W64[(sym ? (int)smem[L.row + f * SP + s] : f) * L.ws64 + k];
+                acc.x += w.x;
+                acc.y += w.y;
+                const float wx = (float)w.x;
+                bx += fabsf(wx);
+                by += fabsf((float)w.y);
+                v = fmaf(wx, wx, v);
+            }
+            base[t] = acc;
+            // non-finite weights give bounds above any limit
+            atomicMax(&mar->bre, __float_as_uint(bx == bx ? bx : 1e30f));
+            atomicMax(&mar->bim, __float_as_uint(by == by ? by : 1e30f));
         }
-        base[t] = acc;
-        // non-finite weights give bounds above any limit
-        atomicMax(&mar->bre, __float_as_uint(bx == bx ? bx : 1e30f));
-        atomicMax(&mar->bim, __float_as_uint(by == by ? by : 1e30f));
+        for (int o = 1; o < kb; o <<= 1) {
+            b += __shfl_xor_sync(kFull, b, o);
+            v += __shfl_xor_sync(kFull, v, o);
+        }
+        const float w = (float)kb, sat = b * (4.f / w) + 8.f * sqrtf(v / w);
+        atomicMax(&mar->sat, __float_as_uint(sat == sat ? sat : 1e30f));
     }
     for (int f = tid >> 5; f <= n; f += nt >> 5) {  // a warp per site
         double acc = 0;
@@ -278,7 +303,10 @@ __device__ inline void load_tables(const SamplerArgs& a, const Layout& L, unsign
         }
     }
     __syncthreads();
-    if (tid == 0) set_margin(*mar, n, m.T, fp64);
+    if (tid == 0) {
+        set_margin(*mar, n, m.T, a.plan.lane_entries, fp64, a.bond_thr24 != 0);
+        if (blockIdx.x == 0) *a.screen_off = mar->off;
+    }
     __syncthreads();
 }
 
@@ -823,6 +851,7 @@ template <int KB, int NG, bool SYM, bool PS, bool F64>
 __global__ void __launch_bounds__(max_threads(KB* NG), 1) screen_kernel(const SamplerArgs a, const Layout L) {
     extern __shared__ __align__(16) unsigned char smem[];
     load_tables(a, L, smem, F64);
+    if (reinterpret_cast<const Margin*>(smem + L.mar)->off) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_warps = (blockDim.x >> 5) * gridDim.x;
     // consecutive chains on different SMs

@@ -72,3 +72,23 @@ def test_fp64_launches_of_one_sweep_equal_one_launch(L, alpha, std):
     kw = dict(n_chains=300, samples_per_chain=10, warmup=3, step=1, bond_flips=0.0, precision=1)
     same(run(L, alpha, std, 0.0, proposal=0, **kw),
          run(L, alpha, std, 0.0, proposal=1, learned_steps=0, learned_train=0, **kw))
+
+
+@pytest.mark.parametrize("precision,chains", [(0, 600), (1, 100)])
+def test_a_launch_left_to_the_sums_and_back(precision, chains):
+    """Persistent chains through captured epochs whose weights the screen takes,
+    then not, then again."""
+    out = []
+    for proposal in (0, 1):
+        cfg = rbmnqs.default_config(rbm_type=1, alpha=4, n_chains=chains, samples_per_chain=3, warmup=0, step=1, seed=5,
+                                    bond_flips=0.0, reinit_chains=0, max_iterations=2, precision=precision,
+                                    proposal=proposal, learned_steps=0, learned_train=0)
+        s = rbmnqs.Session(rbmnqs.Model.kitaev(8), cfg)
+        got = []
+        for std, hid in ((0.02, 0.0), (0.6, 0.0), (0.03, 0.0), (0.02, -9.0), (0.02, 0.5)):
+            s.set_weights(weights(s, std, hid))
+            st, _ = s.epoch()
+            got.append((st["acceptance"], s.sample_configs(), s.spins()))
+        out.append(got)
+    for x, y in zip(*out):
+        same(x, y)

@@ -513,6 +513,12 @@ struct rbmnqs_handle {
             ck(cudaEventRecord(ev[i], st), "event");
     }
 
+    // sweeps of a sampler launch.  Learned proposals: step of them between the
+    // moves, in FP32 by the sums, which keep theta for the moves
+    int launch_sweeps() const {
+        if (cfg.proposal == 1) return fp64 ? std::max(1, cfg.step) : 0;
+        return cfg.warmup + cfg.samples_per_chain * cfg.step;
+    }
     // --- the epoch pieces -------------------------------------------------
     rbmnqs::SamplerArgs sampler_args() const {
         rbmnqs::SamplerArgs a{};
@@ -1358,7 +1364,7 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
         // launch shapes: persistent sampler blocks; evaluation kernels with
         // FP32 W in shared memory when it fits
         ck(rbmnqs::plan_sampler(h->machine(), h->fp64, cfg->n_chains, h->n_prop_bonds, &h->shape, 0, -1,
-                                cfg->proposal == 0),
+                                h->launch_sweeps()),
            "sampler plan");
         if (h->shape.plan.screen && !h->full) {
             h->P32.alloc((size_t)4 * n * nh);
@@ -2174,7 +2180,7 @@ int rbmnqs_autotune(rbmnqs_handle* h, int32_t sweeps, int32_t* sampler_wpb, int3
                 for (int cap = top; cap >= 1; cap /= 2) {
                     rbmnqs::SamplerShape sh{};
                     ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &sh, cap, pm,
-                                            !h->net),
+                                            h->launch_sweeps()),
                        "sampler plan");
                     if (sh.plan.pair != pm) break;  // two chains per warp not possible here
                     if (std::find(tried.begin(), tried.end(), sh.warps_per_block) != tried.end()) continue;
@@ -2192,7 +2198,7 @@ int rbmnqs_autotune(rbmnqs_handle* h, int32_t sweeps, int32_t* sampler_wpb, int3
             }
             rbmnqs::SamplerShape chk{};
             ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &chk,
-                                    best.warps_per_block, best.plan.pair, !h->net),
+                                    best.warps_per_block, best.plan.pair, h->launch_sweeps()),
                "sampler plan");
             h->shape = chk;
         }
@@ -2330,7 +2336,7 @@ int rbmnqs_set_sweep_shape(rbmnqs_handle* h, int32_t warps_per_block, int32_t ch
         require(!h->pf_n, "the Pfaffian buffers are sized for the planned shape", RBMNQS_ERR_UNSUPPORTED);
         rbmnqs::SamplerShape sh{};
         ck(rbmnqs::plan_sampler(h->machine(), h->fp64, h->cfg.n_chains, h->n_prop_bonds, &sh, warps_per_block,
-                                chains_per_warp == 2 ? 1 : 0, !h->net),
+                                chains_per_warp == 2 ? 1 : 0, h->launch_sweeps()),
            "sampler plan");
         require(sh.plan.pair == (chains_per_warp == 2),
                 "two chains per warp needs the FP32 expanded-table sweep with n <= 32", RBMNQS_ERR_UNSUPPORTED);

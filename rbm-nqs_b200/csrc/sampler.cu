@@ -2251,14 +2251,36 @@ static cudaError_t plan_sampler_impl(const MachineDev& m, int fp64, int n_chains
     return cudaSuccess;
 }
 
-// screen false: not the screened sweep for FP32 sessions, whose start (z of every
-// entry) a launch of few sweeps does not earn back (learned moves between
-// sweeps, 8192 chains of 128 spins: 6.8 ms of sweep stage by the exact sums, 8.0
-// screened).
+// Does the screened sweep pay for a launch of `sweeps` sweeps?  Its start (tables, z
+// of every entry) costs 0.2 to 0.7 ms at 512 entries, and its warps are 16 per SM
+// where the sums have up to 28, so it needs chains and sweeps to earn that back.
+// FP32, time over the sums' kernel, 512 entries of 128 spins, Kitaev / toric code /
+// basic machine.  First line: weights of spread 0.035 (5, 30, 15 % accepted), by which
+// the lines are drawn, second: 0.02, untrained (70 % accepted, the screen's worst).
+//   chains per SM, sweeps  64, 1            14, 1            14, 4            7, 16
+//                    0.67 1.08  -     0.80 1.25 0.64   0.54 0.81 0.52   0.68 0.97 0.77
+//                    0.93 1.43  -     1.09 1.58 0.72   0.82 1.22 0.62   1.03 1.38 0.91
+//   and basic machines at 7, 8: 0.83 / 1.04, at 1, 16: 0.90 / 1.02; symmetric ones at
+//   1, 16: 0.93 1.15 / 1.23 1.65.
+// FP64: 0.02 to 0.7, one sweep included, but for the smallest machines' single
+// sweep (8 sites: 1.0 to 1.4).
+static bool screen_pays(const MachineDev& m, int fp64, int n_chains, int sms, int sweeps) {
+    if (fp64) return sweeps > 1 || m.T > 32;
+    const int per_sm = (n_chains + sms - 1) / sms;
+    const int least = per_sm >= 64   ? 1
+                      : per_sm >= 14 ? (m.symmetric ? 4 : 1)
+                      : per_sm >= 4  ? (m.symmetric ? 16 : 8)
+                                     : (m.symmetric ? 32 : 16);
+    return sweeps >= least;
+}
+
 cudaError_t plan_sampler(const MachineDev& m, int fp64, int n_chains, int n_bonds, SamplerShape* out, int max_wpb,
-                         int pair_mode, bool screen) {
-    cudaError_t err = cudaSuccess;
-    if (m.pf.n == 0 && (fp64 || (screen && pair_mode != 1)) &&
+                         int pair_mode, int sweeps) {
+    int dev = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (m.pf.n == 0 && (fp64 || pair_mode != 1) && screen_pays(m, fp64, n_chains, sms, sweeps) &&
         plan_screen(m, fp64, n_chains, n_bonds, max_wpb, out, &err)) {
         if (err != cudaSuccess) return err;
         SamplerShape ex{};
@@ -2376,7 +2398,7 @@ bool sampler_batch_plan(const MachineDev& m, int fp64, int n_chains, int n_bonds
     const int E = elements_per_lane(m.T);
     if (fp64 || m.pf.n > 0 || E > 8) return false;
     SamplerShape sh{};
-    if (plan_sampler(m, 0, n_chains, n_bonds, &sh, kBatchSweepWarps, 0) != cudaSuccess) return false;
+    if (plan_sampler(m, 0, n_chains, n_bonds, &sh, kBatchSweepWarps, 0, 0) != cudaSuccess) return false;
     SmemPlan pl = sh.plan;
     pl.pair = 0;
     if (!pl.use_u && !pl.gather) return false;

@@ -216,9 +216,9 @@ struct SamplerShape : SweepShape {
 };
 // max_wpb > 0 caps the warps per block (launch-shape autotuning); pair_mode
 // 1 asks for two chains per warp where the table path allows it (else, and
-// by default, one chain per warp).
+// by default, one chain per warp).  sweeps: of a launch (0: the sums' kernel).
 cudaError_t plan_sampler(const MachineDev& m, int fp64, int n_chains, int n_bonds, SamplerShape* out,
-                         int max_wpb = 0, int pair_mode = -1, bool screen = true);
+                         int max_wpb, int pair_mode, int sweeps);
 cudaError_t launch_sampler(const SamplerArgs& a, int fp64, const SamplerShape& shape, cudaStream_t st);
 // The sweep screened by products (sampler_screen.cu): its plan (false: not for
 // this machine) and its launch.

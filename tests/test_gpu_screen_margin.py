@@ -92,3 +92,15 @@ def test_a_launch_left_to_the_sums_and_back(precision, chains):
         out.append(got)
     for x, y in zip(*out):
         same(x, y)
+
+
+@pytest.mark.parametrize("warmup,spc,chains,screened", [(0, 1, 16384, True), (0, 1, 2100, False), (2, 1, 2100, False),
+                                                         (3, 1, 2100, True)])
+def test_launches_of_few_sweeps_take_the_sums(warmup, spc, chains, screened):
+    """The launch shape of a session that sweeps by the sums (learned proposals), or not."""
+    shape = []
+    for proposal in (0, 1):
+        cfg = rbmnqs.default_config(rbm_type=1, alpha=4, n_chains=chains, samples_per_chain=spc, warmup=warmup, step=1,
+                                    seed=5, precision=0, proposal=proposal)
+        shape.append(rbmnqs.Session(rbmnqs.Model.kitaev(8), cfg).sweep_shape()[0])
+    assert (shape[0] != shape[1]) == screened

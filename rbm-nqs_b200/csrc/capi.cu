@@ -69,8 +69,15 @@ template <typename T> struct DevBuf {
     size_t n = 0;
     void alloc(size_t count) {
         release();
-        n = count;
-        if (count) ck(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
+        if (count) {
+            const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+            if (e != cudaSuccess) {
+                p = nullptr;
+                cudaGetLastError();  // reported here, not by the next launch
+            }
+            ck(e, "cudaMalloc");
+        }
+        n = count;  // only now: a failed allocation leaves an empty buffer
     }
     void release() {
         if (p) cudaFree(p);

@@ -1752,15 +1752,17 @@ int rbmnqs_set_spins(rbmnqs_handle* h, const uint32_t* spins) {
 
 // Buffers of eval_batch and log_psi_over_psi: one allocation in the handle, kept
 // from call to call up to kEvalKeep bytes (cudaMalloc and cudaFree cost more than
-// a small evaluation) and replaced by one of the call's size above.
-constexpr size_t kEvalKeep = size_t(64) << 20;
+// a small evaluation) and replaced by one of the call's size above.  An FP32 O is
+// widened and copied out kWiden entries at a time, so that a call needs no more
+// memory than its FP32 O and one such piece.
+constexpr size_t kEvalKeep = size_t(64) << 20, kWiden = size_t(2) << 20;
 
 static void eval_common(rbmnqs_handle* h, const uint32_t* spins, int B, double* logpsi, double* eloc, double* O,
                         const int32_t* flips, int nflips, double* ratio) {
     require(h && spins && B >= 0, "bad arguments");
     if (B == 0) return;
     if (ratio) require(flips && nflips >= 1 && nflips <= 6, "1..6 flips per configuration");
-    // one block: spins | complex results | flips | O | FP64 copy of an FP32 O
+    // one block: spins | complex results | flips | O | a piece of an FP32 O in FP64
     const size_t cnt = (size_t)B * h->P, osz = h->osize();
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -1771,7 +1773,7 @@ static void eval_common(rbmnqs_handle* h, const uint32_t* spins, int B, double* 
     const size_t o_s = take((size_t)B * 16), o_l = take(logpsi ? (size_t)B * 16 : 0),
                  o_e = take(eloc ? (size_t)B * 16 : 0), o_r = take(ratio ? (size_t)B * 16 : 0),
                  o_f = take(ratio ? (size_t)B * nflips * sizeof(int) : 0), o_O = take(O ? cnt * osz : 0),
-                 o_D = take(O && !h->fp64 ? cnt * sizeof(double2) : 0);
+                 o_D = take(O && !h->fp64 ? std::min(cnt, kWiden) * sizeof(double2) : 0);
     DevBuf<unsigned char> own;
     if (at > kEvalKeep)
         own.alloc(at);
@@ -1803,13 +1805,16 @@ static void eval_common(rbmnqs_handle* h, const uint32_t* spins, int B, double* 
     if (eloc) ck(cudaMemcpyAsync(eloc, a.eloc, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
     if (ratio) ck(cudaMemcpyAsync(ratio, a.ratio, B * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
     if (O) {
-        const void* src = a.O;
-        if (!h->fp64) {  // widened on the device
-            ck(rbmnqs::launch_widen(static_cast<const float2*>(a.O), cnt, reinterpret_cast<double2*>(base + o_D), h->st),
-               "widen");
-            src = base + o_D;
+        if (h->fp64) {
+            ck(cudaMemcpyAsync(O, a.O, cnt * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
+        } else {  // widened on the device
+            double2* d = reinterpret_cast<double2*>(base + o_D);
+            for (size_t i = 0; i < cnt; i += kWiden) {
+                const size_t k = std::min(kWiden, cnt - i);
+                ck(rbmnqs::launch_widen(static_cast<const float2*>(a.O) + i, k, d, h->st), "widen");
+                ck(cudaMemcpyAsync(O + 2 * i, d, k * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
+            }
         }
-        ck(cudaMemcpyAsync(O, src, cnt * sizeof(double2), cudaMemcpyDeviceToHost, h->st), "c");
     }
     ck(cudaStreamSynchronize(h->st), "sync");
 }

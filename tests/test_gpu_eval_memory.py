@@ -1,5 +1,5 @@
-"""eval_batch's device memory: an allocation that fails leaves the session as it
-was."""
+"""eval_batch's device memory: an FP32 O leaves in pieces, and an allocation that
+fails leaves the session as it was."""
 import numpy as np
 import pytest
 
@@ -19,6 +19,15 @@ def session(alpha=4, precision=0):
 
 def spins(B):
     return O.random_spins(np.random.default_rng(2), B, 32)
+
+
+def test_log_derivatives_in_pieces():
+    """40001 x 133 entries: two pieces of 2^21 and a remainder."""
+    s = session()
+    c = spins(40001)
+    _, _, a = s.eval_batch(c, logpsi=False, eloc=False)
+    for r in (slice(0, 100), slice(15700, 15900), slice(31500, 31600), slice(39990, 40001)):
+        assert np.array_equal(a[r], s.eval_batch(c[r], logpsi=False, eloc=False)[2])
 
 
 def test_failed_allocation_leaves_the_session_usable():

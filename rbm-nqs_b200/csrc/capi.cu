@@ -1285,8 +1285,12 @@ int rbmnqs_create(const rbmnqs_model* mdl, const rbmnqs_config* cfg, rbmnqs_hand
         }
         h->multi_cg = h->mfree && cfg->solver == 0;
         // O of a basic RBM has rank-one blocks (spins x activations); the
-        // Pfaffian columns and the centred O of full enumeration do not
-        h->fact_cg = h->multi_cg && cfg->rbm_type == 0 && !h->pf_n && !h->full && h->n <= 128;
+        // Pfaffian columns and the centred O of full enumeration do not.  A small
+        // FP32 O in L2 is as quick to stream (us per iteration, factors / O: 64
+        // samples x 2600 parameters 18.2 / 17.0, x 2144 18.0 / 17.9; x 4256 18.6 /
+        // 22.1, 256 x 2144 17.7 / 21.5; FP64 64 x 2144 19.4 / 20.7)
+        h->fact_cg = h->multi_cg && cfg->rbm_type == 0 && !h->pf_n && !h->full && h->n <= 128 &&
+                     (h->fp64 || (double)h->N * h->P >= 2e5);
         if (h->mfree || h->coop_dense) {
             const int nn = h->mfree ? h->N : 1;
             ck(rbmnqs::mfree_plan(nn, h->P, &h->mfp), "cooperative CG plan");

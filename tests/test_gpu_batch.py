@@ -92,3 +92,27 @@ def test_autotune_sr_keeps_S_within_tolerance():
     for _ in range(2):
         st, sr = a.epoch()
         assert sr["status"] == 0
+
+
+def test_small_matrix_free_systems_share_a_launch():
+    """A basic machine's FP32 system too small to gain by its factors joins the
+    other matrix-free systems' launch, with the same results."""
+    def make_pair():
+        out = []
+        for pf in (0, 1):
+            cfg = rbmnqs.default_config(rbm_type=0, alpha=2, n_chains=64, samples_per_chain=1, warmup=2, seed=4,
+                                        precision=0, max_iterations=30, pfaffian=pf)
+            s = rbmnqs.Session(rbmnqs.Model.kitaev(4), cfg)
+            rng = np.random.default_rng(pf)
+            s.set_weights(0.05 * (rng.normal(size=s.n_params) + 1j * rng.normal(size=s.n_params)))
+            out.append(s)
+        return out
+    a, b = make_pair(), make_pair()
+    batch = rbmnqs.Batch(a)
+    for _ in range(2):
+        batch.epoch()
+        for s in b:
+            s.epoch()
+    for x, y in zip(a, b):
+        assert np.array_equal(x.get_weights(), y.get_weights())
+    assert batch.graph_kernels() == sum(s.graph_kernels() for s in b) - 2

@@ -2308,9 +2308,9 @@ cudaError_t ensure_dynamic_smem(const void* fn, int bytes) {
 }
 
 // The FP32 expanded-table (one chain per warp) and gather paths store
-// theta_out; the FP64, Pfaffian and two-chain paths do not.
+// theta_out; the FP64, screened, Pfaffian and two-chain paths do not.
 bool sampler_writes_theta(const MachineDev& m, int fp64, const SamplerShape& sh) {
-    return !fp64 && m.pf.n == 0 && !sh.plan.pair && (sh.plan.screen || sh.plan.use_u || sh.plan.gather);
+    return !fp64 && m.pf.n == 0 && !sh.plan.pair && !sh.plan.screen && (sh.plan.use_u || sh.plan.gather);
 }
 
 cudaError_t launch_sampler(const SamplerArgs& a0, int fp64, const SamplerShape& sh, cudaStream_t st) {

@@ -64,9 +64,6 @@ bool plan_screen(const MachineDev& m, int fp64, int n_chains, int n_bonds, int m
     pl.screen = 1;
     pl.lane_entries = elements_per_lane(m.T);
     pl.p_budget = kBasicRows;
-    // machines whose learned moves hand theta back to the sweep
-    pl.lane_rows = m.symmetric && 32 % m.nh == 0 && m.T == 32 * pl.lane_entries && pl.lane_entries >= 4 &&
-                   (m.n + 1) * m.T * 8 > 64 * 1024;
     out->plan = pl;
     out->warps_per_block = wpb;
     out->blocks = (int)blocks;

@@ -604,22 +604,12 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
     const uint32_t thr = a.bond_thr24;
     volatile float hold[8 * NP];  // z, then z p of the open proposal
     bool open = false;            // the loop left at a proposal that needs the exact sums
-    for (;;) {
+    for (; total > 0;) {
         if (!open) {
-            // the start of sweep st with theta wanted: z from theta, or theta
-            // of the final configuration
-            const int st = S->st;
+            // z from theta at the start of the sweep
             if (lane < 4) S->start[lane] = S->sp[lane];
             __syncwarp();
-            if (!F64 && st == 0 && a.theta_in && a.plan.lane_rows) {
-                const float2* src = a.theta_in + (size_t)chain * 32 * a.plan.lane_entries;
-                if constexpr (!F64)
-                    for (int t = lane; t < T; t += 32) th[t] = src[t];
-                __syncwarp();
-            } else {
-                theta_of();
-            }
-            if (st == total) break;
+            theta_of();
             float2 zr[NP], zi[NP];
 #pragma unroll
             for (int j = 0; j < NG; j++) {
@@ -830,13 +820,7 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
             S->k = k;
         }
         __syncwarp();
-        if (!open && st == total && !a.theta_out) break;
-    }
-    if (a.theta_out) {
-        // FP32 theta of the final configuration, zero beyond T
-        const int TP = 32 * a.plan.lane_entries;
-        float2* dst = a.theta_out + (size_t)chain * TP;
-        for (int t = lane; t < TP; t += 32) dst[t] = t < T ? th32[t] : make_float2(0.f, 0.f);
+        if (!open && st == total) break;
     }
     const uint32_t sp[4] = {S->sp[0], S->sp[1], S->sp[2], S->sp[3]};
     chain_finish(a, chain, lane, sp, S->nacc, S->prop);

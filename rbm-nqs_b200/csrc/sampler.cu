@@ -1435,7 +1435,8 @@ template <int E, typename R, int FAST, bool PF>
 __global__ void __launch_bounds__(FAST == 2 ? MaxThreads<E, PF>::gather
                                             : (FAST == 3 ? MaxThreads<E, PF>::pair : MaxThreads<E, PF>::v),
                                   1) sampler_kernel(const SamplerArgs a) {
-    if (a.gate && !*a.gate) return;
+    if constexpr (!PF && FAST != 3)  // behind a screened sweep
+        if (a.gate && !*a.gate) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int fp64 = sizeof(R) == 8;
     Smem sm = carve(smem, a.m, fp64, a.plan, a.n_prop_bonds, sweep_warp_bytes(a.m.T, sizeof(R), PF));

@@ -604,12 +604,14 @@ __device__ __forceinline__ void run_chain(const SamplerArgs& a, const Layout& L,
     const uint32_t thr = a.bond_thr24;
     volatile float hold[8 * NP];  // z, then z p of the open proposal
     bool open = false;            // the loop left at a proposal that needs the exact sums
-    for (; total > 0;) {
+    for (;;) {
         if (!open) {
             // z from theta at the start of the sweep
+            const int st = S->st;
             if (lane < 4) S->start[lane] = S->sp[lane];
             __syncwarp();
             theta_of();
+            if (st >= total) break;  // a launch of no sweeps
             float2 zr[NP], zi[NP];
 #pragma unroll
             for (int j = 0; j < NG; j++) {

@@ -37,13 +37,15 @@
 //
 // Layout as in eloc.cuh: groups of KB hidden units with one symmetry index s,
 // lane l owns the groups l + 32 j; entries in pairs, real and imaginary parts
-// apart.  Bound: shared-memory wavefronts (ncu: 82 % of peak; 10.9 thousand per
-// configuration of 128 spins and 512 entries, 4.9 of them the q rows, 4.3 the
-// FP64 recompute of theta), the FMA pipe at 32 %, issue 51 %.  Measured on 262144
-// configurations of 128 spins, 512 entries, with O_k: 29.6 ms by ln cosh sums
-// (eloc.cuh, which stays for basic machines, whose flipped rows are not shared,
-// and for tables beyond shared memory), 14.2 ms here; 4096 of 32 spins, 128
-// entries: 0.061 and 0.053 ms.
+// apart.  Bound: shared-memory wavefronts (ncu: 82 % of peak, 86 % with O_k; 10.9
+// thousand per configuration of 128 spins and 512 entries, 4.9 of them the q rows,
+// 4.3 the FP64 recompute of theta, and 2.5 for O_k), the FMA pipe at 35 %, issue
+// 53 %.  Measured on 262144 configurations of 128 spins, 512 entries, with O_k: 29.3
+// ms by ln cosh sums (eloc.cuh, which stays for basic machines, whose flipped rows
+// are not shared, and for tables beyond shared memory), 13.9 ms here; 4096 of 32
+// spins, 128 entries: 0.061 and 0.055 ms.  8192 of 128 spins whose products are all
+// rescaled (weights of spread 0.3) 1.03 ms, as by ln cosh sums; all in ratio_slow()
+// 10 ms.
 #include <algorithm>
 #include <map>
 #include <mutex>

@@ -13,8 +13,9 @@
 // configuration after every sweep (mixed-precision scheme), so FP32
 // drift never outlives one sweep.  With the Pfaffian factor (sites <= 32) the
 // warp also holds X^{-1} in shared memory (pfaffian.cuh).  FP64 sweeps, and FP32
-// sweeps of 16 entries per lane, screen the proposals by products
-// (sampler_screen.cuh).
+// sweeps of 16 entries per lane in launches of enough chains and sweeps
+// (screen_pays), screen the proposals by products (sampler_screen.cuh), whose drift
+// the screen's margin allows for.
 #include <algorithm>
 #include <map>
 #include <mutex>

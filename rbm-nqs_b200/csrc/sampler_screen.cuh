@@ -49,28 +49,31 @@
 // estimate, m0 + coef (a^2 + b^2) with m0 = 8e-4 + 1e-4 max |Re theta| and coef = 2e-6
 // + 5e-7 max |Im theta|.  Over 5e7 proposals of machines of 384 and 512 entries
 // (weights of spread 0.005 to 0.1, hidden biases of either sign, near the zeros of
-// cosh, all entries of a unit equal) the largest difference was 0.29 of it, and the
-// screen's error against 64 bits below the sums' own.  A decision beyond it would
-// be one between two FP32 values of a tie, as the sums' decisions of ties are.
+// cosh, all entries of a unit equal) the largest difference was 0.29 of it.  Against
+// 64 bits the screen was off by 2.4e-4 at most, so what it decides is right by them
+// too; chains, samples and counters are those of the FP32 sums, bit for bit, in every
+// test.
 //
 // Weights that leave too many proposals open (kOff: the FP64 margin at mean counts
 // and |1 + z| = 1), that reach |Re theta| > 40, that mostly overflow a product of four
 // |1 + z|^2 (a sum of -Re theta of 22; 512 entries of 128 spins: spread of the weights
-// 0.2 0.2 % of the proposals, 0.25 48 %, 0.3 94 %), or that FP32 factors do not hold, turn the launch over
-// to the sums' kernel (sampler.cu), which is launched behind this one and returns at
-// once otherwise.
+// 0.2 0.2 % of the proposals, 0.25 48 %, 0.3 94 %), or that FP32 factors do not hold,
+// turn the launch over to the sums' kernel (sampler.cu), which is launched behind
+// this one and returns at once otherwise (2 us).  At a spread of 0.3, 16384 chains x 4
+// sweeps: 17.9 ms screened, 5.0 by the sums.
 //
 // Layout: groups of KB consecutive hidden units with one symmetry index, lane l
 // owns the groups l + 32 j, entries in pairs (packed FP32x2).  Symmetric machines
 // keep p and W of every row in shared memory and find the row of (site, symmetry)
 // in a 16-bit table; basic machines read row f directly, from shared memory or,
 // where p does not fit, from L2.  The loop is bound by issue and latency (ncu, 512
-// entries: 330 warp instructions a proposal, issue 64 % of active cycles, LSU 39 %,
-// FMA pipe 36 %, FP64 2 %; 16 warps at 128 registers: with 20 at 96 the loop
+// entries: 327 warp instructions a proposal, issue 62 % of active cycles, LSU 42 %,
+// FMA pipe 34 %, FP64 1.5 %; 16 warps at 128 registers: with 20 at 96 the loop
 // spills, 15.8 ms below).  Measured: 16384 chains x 16 sweeps of 128 spins, 512
-// entries, FP32: 19.8 ms by the exact sums, 13.7 screened, 0.12 % of the proposals
-// decided exactly; FP64 sessions, 500 chains x 19 sweeps of 32 spins, 96 entries:
-// 1.32 ms by the sums, 0.22 screened.
+// entries, FP32: 19.7 ms by the exact sums, 14.1 screened, 0.17 % of the proposals
+// decided exactly (28 ms with a worst case of the FP32 sums' rounding in the margin);
+// FP64 sessions, 500 chains x 19 sweeps of 32 spins, 96 entries: 1.33 ms by the sums,
+// 0.25 screened (0.22 with FP32's margin), 0.8 % decided exactly.
 #pragma once
 
 #include <type_traits>
